@@ -666,7 +666,8 @@ struct __align__(16) RaySample {
   float tx, ty, tz;          // transmittance texel -> sample x dx x trapezoid weight
   float d;                   // distance from the texel's point along its ray
   float inv_r;               // 1 / r at the sample
-  float pad[3];
+  float pad;
+  float rb_inv_r, rb_d;      // Rb / r and Rb d / r at the sample
 };
 
 struct MultipleFastDims {
@@ -686,18 +687,6 @@ __host__ __device__ inline MultipleFastDims MultipleDims(const Shape& s) {
   if (s.tune[1] > 0) group = s.tune[1];
   return MultipleFastDims{rows, group};
 }
-bool MultipleFastFits(const Shape& s) {
-  return s.sw() <= kMultipleFastThreads * kMultipleFastMaxCols;
-}
-int MultipleFastTiles(const Shape& s) {
-  const int rows = MultipleDims(s).rows;
-  return (s.sr * s.smu + rows - 1) / rows;
-}
-int MultipleFastSmem(const Shape& s) {
-  const MultipleFastDims d = MultipleDims(s);
-  return d.rows * kRaySamples * (int)sizeof(RaySample) + 2 * d.group * d.rows * s.sw() * 16;
-}
-
 // The LUT row that logical row i of the multiple-scattering blocks takes.
 __device__ __forceinline__ int RowAt(const Tables& tab, int i) {
   return tab.row_order ? __ldg(tab.row_order + i) : i;
@@ -741,7 +730,9 @@ __device__ RaySample MakeRaySample(const Instance& in, int rowi, int i) {
   rs.tz = t.z * dw;
   rs.d = d;
   rs.inv_r = 1.0f / p.r;
-  rs.pad[0] = rs.pad[1] = rs.pad[2] = 0.0f;
+  rs.rb_inv_r = c.Rb / p.r;
+  rs.rb_d = rs.rb_inv_r * d;
+  rs.pad = 0.0f;
   return rs;
 }
 
@@ -928,11 +919,367 @@ __device__ __forceinline__ void MultipleFastBlock(const Instance& in, int local,
   }
 }
 
+// ---------------------------------------------------------------------------
+// Multiple scattering by nu nodes (MultipleKind 1 and 2): no shared line.
+//
+// The columns of one nu node's block are the MU_S <= 64 mu_s columns of that
+// node, so a warp can hold a sample's interpolated line of one node (two
+// columns per lane above MU_S = 32) or of several nodes (32 / MU_S) in
+// registers: a lane interpolates its own columns from the four delta-density
+// rows, and a texel's two mu_s taps are shuffles.  A warp then marches the 51
+// samples of a row on its own, with no line in shared memory and no barrier
+// per line stage.
+//
+// A texel whose nu is not clamped sits on its own node, so its taps are in
+// its own warp.  The texels of a row and column whose nu is clamped share the
+// clamped value (one below, one above the physical range), which lies between
+// two nodes n0, n0 + 1: the lanes of column c in those two nodes' warps each
+// march that nu through their own node's line, weighted with the node's lerp
+// weight, and the two parts are added through shared memory at the end.  A
+// lane's work is thus up to three of {its own texel, the low and the high
+// clamped nu}, put in up to three slots; a slot is marched when any lane of
+// the warp uses it (1.7 of them on average at the reference's shape).
+//
+// Bound by instruction issue (70%) and the L1 data pipe (75%) together: 111
+// instructions and 31 wavefronts per warp and sample, against 135 and 45 of
+// the lines in shared memory, whose stores, taps and clamps it does without.
+// Per 16-instance launch at the reference's shape 4.13 -> 3.26 ms; one
+// high-resolution instance 4.40 -> 3.37 ms.
+// ---------------------------------------------------------------------------
+constexpr int kNodeWarps = kMultipleFastThreads / 32;
+__host__ __device__ inline bool MultipleByNodes(const Shape& s) { return MultipleKind(s) < 4; }
+// Nu nodes held by one warp, and warp items (of that many nodes) per row.
+__host__ __device__ inline int NodesPerWarp(const Shape& s) {
+  return s.smus <= 32 ? 32 / s.smus : 1;
+}
+__host__ __device__ inline int NodeItemsPerRow(const Shape& s) {
+  const int per = NodesPerWarp(s);
+  return (s.snu + per - 1) / per;
+}
+// Rows per block: as many (up to 4) as give its 8 warps one item each, or two
+// where that leaves two full waves of blocks (4 per SM on 152 SMs).  Two items
+// per warp halve the blocks' idle time (their sample tables are built by 51
+// threads per row, and the warps of the outermost nodes have less to do):
+// 3.26 ms per 16-instance launch at the reference's shape against 3.37 with
+// one (four give 3.22 but too few blocks for a single instance); smaller LUTs
+// want the shorter blocks.
+__host__ __device__ inline int NodeRows(const Shape& s) {
+  const int items = NodeItemsPerRow(s);
+  const bool many = (long long)s.sr * s.smu * items >= 2LL * 2 * kNodeWarps * 4 * 152;
+  const int rows = (many ? 2 : 1) * kNodeWarps / items;
+  return rows < 1 ? 1 : (rows > 4 ? 4 : rows);
+}
+
+// The mu_s mapping along a ray: with a = (d - d_min) / (d_max - d_min) the
+// mapping's x = (1 - a / A) / (1 + a) is ((A + 1) / (1 + a) - 1) / A, one FMA
+// of 1 / (1 + a).
+struct SunMap {
+  float H2, c0, c1, c1h2;   // 1 + a = c0 + c1 d; c1 H^2
+  float k1, k0;             // x = k1 / (1 + a) + k0, clamped to [0, 1]
+  float n1;                 // MU_S - 1
+};
+__device__ __forceinline__ SunMap MakeSunMap(const Consts& c, const Shape& s) {
+  SunMap m;
+  const float d_min = c.Rt - c.Rb, inv_A = 1.0f / c.mus_A;
+  m.H2 = c.H * c.H;
+  m.c1 = 1.0f / (c.H - d_min);
+  m.c0 = 1.0f - d_min * m.c1;
+  m.c1h2 = m.c1 * m.H2;
+  m.k1 = 1.0f + inv_A;
+  m.k0 = -inv_A;
+  m.n1 = float(s.smus - 1);
+  return m;
+}
+// The mapping's x, in [0, 1], where the sun's cosine is rmus / Rb.
+__device__ __forceinline__ float SunCoordinate(const SunMap& m, float rmus) {
+  // H^2 + rmus^2 >= H^2 and y >= H: normal.  d = H^2 / y above the horizon,
+  // y below it (cancellation-free), so 1 / (1 + a) is y / (c0 y + c1 H^2) or
+  // 1 / (c0 + c1 y), both denominators >= min(1, H).
+  const float y = SqrtFtz(fmaf(rmus, rmus, m.H2)) + fabsf(rmus);
+  const bool up = rmus > 0.0f;
+  const float q = DivFtz(up ? y : 1.0f, fmaf(up ? m.c0 : m.c1, y, up ? m.c1h2 : m.c0));
+  return FmaSat(q, m.k1, m.k0);
+}
+
+// A 256-bit read-only load of two neighbouring texels (32-byte aligned).
+__device__ __forceinline__ void LoadTwo(float4& a, float4& b, const float4* ptr) {
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+      : "l"(ptr));
+}
+
+// A lane's columns of one LUT row: one, two with a 256-bit load (kPair: the
+// columns are 32-byte aligned), or two loads (second: the offset of the
+// second column, 0 where the lane has one).
+template <int kCols>
+struct NodeRow {
+  float4 v[kCols];
+};
+template <int kCols, bool kPair>
+__device__ __forceinline__ void LoadRow(NodeRow<kCols>& row, const float4* col, int offset,
+                                        int second, [[maybe_unused]] long long n) {
+  if constexpr (kCols == 1) {
+    row.v[0] = __ldg(ATMO_LINE_PTR(col, offset, 0, n));
+  } else if constexpr (kPair) {
+    LoadTwo(row.v[0], row.v[1], ATMO_LINE_PTR(col, offset, 0, n - 1));
+  } else {
+    row.v[0] = __ldg(ATMO_LINE_PTR(col, offset, 0, n));
+    row.v[1] = __ldg(ATMO_LINE_PTR(col, offset, second, n));
+  }
+}
+
+__device__ __forceinline__ F3 Shuffle3(F3 v, int lane) {
+  return F3{__shfl_sync(0xffffffffu, v.x, lane), __shfl_sync(0xffffffffu, v.y, lane),
+            __shfl_sync(0xffffffffu, v.z, lane)};
+}
+
+// The line at x of the mu_s range of the lane's node.  magic: kRoundMagic
+// plus the node's first lane; the FMA rounded down leaves the lower tap's
+// lane in the sum's low bits (a shuffle's lane counts modulo 32: at x = 1 the
+// upper tap, of weight 0, may be any lane).
+template <int kCols>
+__device__ __forceinline__ F3 TapLine(const F3 (&line)[kCols], float x, float n1, float magic) {
+  const float t = __fmaf_rd(x, n1, magic);
+  const float w1 = fmaf(x, n1, magic - t), w0 = 1.0f - w1;
+  const int i0 = __float_as_int(t);
+  if constexpr (kCols == 1) {
+    const F3 t0 = Shuffle3(line[0], i0), t1 = Shuffle3(line[0], i0 + 1);
+    return fma3(t1, w1, t0 * w0);
+  } else {
+    // Columns 2 l, 2 l + 1 in lane l: the taps i0, i0 + 1 are one even and
+    // one odd column.
+    const bool odd = i0 & 1;
+    const F3 te = Shuffle3(line[0], (i0 + 1) >> 1), to = Shuffle3(line[1], i0 >> 1);
+    return fma3(to, odd ? w0 : w1, te * (odd ? w1 : w0));
+  }
+}
+
+// Marches the row's samples: acc[s][m] += the line's value at the nu of slot
+// s of the lane's column m, times the sample's transmittance and weight.
+template <int kCols, int kSlots, bool kPair>
+__device__ __forceinline__ void MarchNodes(const RaySample* samp, const float4* col, int second,
+                                           long long n, const SunMap& map, float magic,
+                                           const float (&rmu_s)[kCols],
+                                           const float (&nu)[kSlots][kCols],
+                                           F3 (&acc)[kSlots][kCols]) {
+  NodeRow<kCols> a, b, p, q;
+  int4 r = *reinterpret_cast<const int4*>(&samp[0].r00);
+  LoadRow<kCols, kPair>(a, col, r.x, second, n);
+  LoadRow<kCols, kPair>(b, col, r.y, second, n);
+  LoadRow<kCols, kPair>(p, col, r.z, second, n);
+  LoadRow<kCols, kPair>(q, col, r.w, second, n);
+#pragma unroll 1
+  for (int i = 0; i < kRaySamples; ++i) {
+    const float4 w = *reinterpret_cast<const float4*>(&samp[i].w00);
+    F3 line[kCols];
+#pragma unroll
+    for (int m = 0; m < kCols; ++m) {
+      line[m] = fma3(f3(q.v[m]), w.w,
+                     fma3(f3(p.v[m]), w.z, fma3(f3(b.v[m]), w.y, f3(a.v[m]) * w.x)));
+    }
+    // The next sample's rows are loaded while this one's taps are made; a
+    // sample in the same cell (r00 and r11 fix all four rows) keeps them.
+    if (i + 1 < kRaySamples) {
+      const int4 r1 = *reinterpret_cast<const int4*>(&samp[i + 1].r00);
+      if (r1.x != r.x || r1.w != r.w) {
+        LoadRow<kCols, kPair>(a, col, r1.x, second, n);
+        LoadRow<kCols, kPair>(b, col, r1.y, second, n);
+        LoadRow<kCols, kPair>(p, col, r1.z, second, n);
+        LoadRow<kCols, kPair>(q, col, r1.w, second, n);
+        r = r1;
+      }
+    }
+    // Rb mu_s at the sample: (r mu_s + d nu) Rb / r_i.
+    const float3 t{samp[i].tx, samp[i].ty, samp[i].tz};
+    const float2 rb = *reinterpret_cast<const float2*>(&samp[i].rb_inv_r);
+#pragma unroll
+    for (int m = 0; m < kCols; ++m) {
+      const float rmus = rmu_s[m] * rb.x;
+#pragma unroll
+      for (int s = 0; s < kSlots; ++s) {
+        const float x = SunCoordinate(map, fmaf(nu[s][m], rb.y, rmus));
+        acc[s][m] = fma3(TapLine<kCols>(line, x, map.n1, magic), F3{t.x, t.y, t.z}, acc[s][m]);
+      }
+    }
+  }
+}
+
+// The nu of a texel and whether it sits on its own node (MakeAngles).  Not
+// inlined: the lanes that march a clamped nu and the texels that take the sum
+// must agree on which texels are clamped, to the bit.
+struct NodeNu {
+  float nu;
+  int side;   // -1 on the texel's own node, 0 clamped from below, 1 from above
+};
+__device__ __noinline__ NodeNu TexelNu(const Instance& in, int rowi, int col, int n) {
+  const TexelAngles a = MakeAngles(in.s, in.tab.rows[rowi], in.tab.cols[col], n);
+  return NodeNu{a.nu, a.on_node ? -1 : a.raised ? 0 : 1};
+}
+
+// Adds a texel's result to the LUTs (functions.glsl:1369-1383).
+__device__ __forceinline__ void StoreMultiple(const Instance& in, int texel, F3 sum, float nu) {
+  [[maybe_unused]] const long long nS = in.s.s_texels();
+  texel = (int)ATMO_CHECKED_INDEX(kCheckOutput, texel, nS);
+  in.dR[texel] = to4(sum, 1.0f);   // delta multiple aliases delta Rayleigh
+  const F3 add = MatVec(in.c.lum, sum) * (1.0f / RayleighPhase(in.c, nu));
+  const float4 o = in.S[texel];
+  in.S[texel] = make_float4(o.x + add.x, o.y + add.y, o.z + add.z, o.w);
+}
+
+template <int kCols, bool kPair>
+__device__ __forceinline__ void MultipleNodesBlock(const Instance& in, int local, float4* smem) {
+  const Shape s = in.s;
+  const Consts& c = in.c;
+  const int W = s.sw(), R = NodeRows(s), per = NodesPerWarp(s), items = NodeItemsPerRow(s);
+  const int rows_total = s.sr * s.smu, row0 = local * R;
+  [[maybe_unused]] const long long nS = s.s_texels();   // checked build
+  RaySample* samp = reinterpret_cast<RaySample*>(smem);                        // [R][51]
+  float4* edge = smem + R * kRaySamples * (int)(sizeof(RaySample) / 16);       // [R][2][2][MU_S]
+  const int lane = threadIdx.x & 31, warp = threadIdx.x / 32;
+
+  for (int e = threadIdx.x; e < R * kRaySamples; e += kMultipleFastThreads) {
+    const int rr = e / kRaySamples, i = e - rr * kRaySamples;
+    if (row0 + rr < rows_total) samp[e] = MakeRaySample(in, RowAt(in.tab, row0 + rr), i);
+  }
+  for (int e = threadIdx.x; e < R * 4 * s.smus; e += kMultipleFastThreads)
+    edge[e] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  __syncthreads();
+
+  const SunMap map = MakeSunMap(c, s);
+  const float nodes1 = float(s.snu - 1);
+  for (int item = warp; item < R * items; item += kNodeWarps) {
+    const int rr = item / items;
+    if (row0 + rr >= rows_total) break;
+    // Rotated from row to row: the outermost nodes have the least work.
+    const int slot = (item + 3 * rr) % items;
+    const int rowi = RowAt(in.tab, row0 + rr);
+    const int sub = kCols == 1 ? lane / s.smus : 0;
+    const int n = slot * per + sub;
+    const int col0 = kCols == 1 ? lane - sub * s.smus : 2 * lane;
+    const int cols = sub < per && n < s.snu ? min(max(s.smus - col0, 0), kCols) : 0;
+    // Lanes without a texel march column 0 of node 0 and keep nothing.
+    const int second = cols == 2 ? 1 : 0;
+    const float4* col = in.dJ + (cols > 0 ? n * s.smus + col0 : 0);
+    float rmu_s[kCols], nu[3][kCols], weight[3][kCols];
+    int use[3][kCols], slots = 0;   // 0: none, 1: own texel, 2 + 2 side + half: clamped part
+#pragma unroll
+    for (int m = 0; m < kCols; ++m) {
+      const int colm = m < cols ? col0 + m : 0;
+      const NodeNu own = TexelNu(in, rowi, colm, min(n, s.snu - 1));
+      rmu_s[m] = in.tab.rows[rowi].r * in.tab.cols[colm].mu_s;
+      int used = 0;
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        nu[q][m] = own.nu;
+        weight[q][m] = 1.0f;
+        use[q][m] = 0;
+      }
+      if (m < cols && own.side < 0) {
+        use[0][m] = 1;
+        used = 1;
+      }
+#pragma unroll
+      for (int side = 0; side < 2; ++side) {
+        const NodeNu end = TexelNu(in, rowi, colm, side == 0 ? 0 : s.snu - 1);
+        const float x = (end.nu + 1.0f) * 0.5f * nodes1, fx = floorf(x);
+        const int half = n - (int)fx;   // 0: the lower of the two nodes, 1: the upper
+        const float l1 = x - fx;
+        // Some texel's nu is clamped at an end where the end node's own is.
+        if (m < cols && end.side == side && (half == 0 || half == 1)) {
+          const float w = half == 0 ? 1.0f - l1 : l1;
+#pragma unroll
+          for (int q = 0; q < 3; ++q) {
+            if (q == used) {
+              nu[q][m] = end.nu;
+              weight[q][m] = w;
+              use[q][m] = 2 + 2 * side + half;
+            }
+          }
+          ++used;
+        }
+      }
+      slots = max(slots, used);
+    }
+    slots = __reduce_max_sync(0xffffffffu, slots);
+    const RaySample* srow = samp + rr * kRaySamples;
+    const float magic = kRoundMagic + (kCols == 1 ? float(sub * s.smus) : 0.0f);
+    auto keep = [&](int m, int used, float w, float nu_m, F3 sum) {
+      if (used == 1) StoreMultiple(in, rowi * W + n * s.smus + col0 + m, sum, nu_m);
+      if (used >= 2) {
+        edge[(rr * 4 + used - 2) * s.smus + col0 + m] = to4(sum * w, 0.0f);
+      }
+    };
+    for (int first = 0; first < slots; first += 2) {
+      float nu2[2][kCols];
+      F3 acc[2][kCols];
+#pragma unroll
+      for (int m = 0; m < kCols; ++m) {
+        nu2[0][m] = first == 0 ? nu[0][m] : nu[2][m];
+        nu2[1][m] = nu[1][m];
+        acc[0][m] = acc[1][m] = f3(0.0f);
+      }
+      if (slots - first >= 2) {
+        MarchNodes<kCols, 2, kPair>(srow, col, second, nS, map, magic, rmu_s, nu2, acc);
+      } else {
+        float nu1[1][kCols];
+        F3 acc1[1][kCols];
+#pragma unroll
+        for (int m = 0; m < kCols; ++m) {
+          nu1[0][m] = nu2[0][m];
+          acc1[0][m] = f3(0.0f);
+        }
+        MarchNodes<kCols, 1, kPair>(srow, col, second, nS, map, magic, rmu_s, nu1, acc1);
+#pragma unroll
+        for (int m = 0; m < kCols; ++m) acc[0][m] = acc1[0][m];
+      }
+#pragma unroll
+      for (int m = 0; m < kCols; ++m) {
+        keep(m, first == 0 ? use[0][m] : use[2][m], first == 0 ? weight[0][m] : weight[2][m],
+             nu2[0][m], acc[0][m]);
+        if (first == 0) keep(m, use[1][m], weight[1][m], nu2[1][m], acc[1][m]);
+      }
+    }
+  }
+  __syncthreads();
+
+  // The clamped texels: the sum of their two nodes' parts.
+  for (int e = threadIdx.x; e < R * W; e += kMultipleFastThreads) {
+    const int rr = e / W, x = e - rr * W;
+    if (row0 + rr >= rows_total) break;
+    const int rowi = RowAt(in.tab, row0 + rr);
+    const int n = x / s.smus, colx = x - n * s.smus;
+    const NodeNu ang = TexelNu(in, rowi, colx, n);
+    if (ang.side < 0) continue;
+    const float4 u = edge[(rr * 4 + 2 * ang.side) * s.smus + colx];
+    const float4 v = edge[(rr * 4 + 2 * ang.side + 1) * s.smus + colx];
+    StoreMultiple(in, rowi * W + x, F3{u.x + v.x, u.y + v.y, u.z + v.z}, ang.nu);
+  }
+}
+
+// MultipleKind 1 (kCols 1; 64 registers, 4 blocks per SM) and 2 (kCols 2;
+// 128 registers, 2 blocks per SM: 3 at 80 registers spill and run 1% slower).
+// An instance is always marched by the same kernel, whatever shapes share its
+// launch: the blocks of the other instances return at once.
+template <int kCols>
+__global__ void __launch_bounds__(kMultipleFastThreads, kCols == 1 ? 4 : 2)
+k_multiple_nodes(const Instance* __restrict__ insts, WorkList wl) {
+  extern __shared__ float4 smem[];
+  int local;
+  const Instance& in = insts[FindEntry(wl, blockIdx.x, &local)];
+  if (MultipleKind(in.s) != kCols) return;
+  if (kCols == 2 && in.s.smus % 2 == 0 && ((size_t)in.dJ & 31) == 0) {
+    MultipleNodesBlock<kCols, kCols == 2>(in, local, smem);
+  } else {
+    MultipleNodesBlock<kCols, false>(in, local, smem);
+  }
+}
+
 __global__ void __launch_bounds__(kMultipleFastThreads, 4)
 k_multiple_fast(const Instance* __restrict__ insts, WorkList wl) {
   extern __shared__ float4 smem[];
   int local;
   const Instance& in = insts[FindEntry(wl, blockIdx.x, &local)];
+  if (MultipleKind(in.s) != 4) return;
   if (in.s.sw() <= kMultipleFastThreads) {
     MultipleFastBlock<1>(in, local, smem);
   } else {
@@ -940,10 +1287,27 @@ k_multiple_fast(const Instance* __restrict__ insts, WorkList wl) {
   }
 }
 
+bool MultipleFastFits(const Shape& s) {
+  return MultipleByNodes(s) || s.sw() <= kMultipleFastThreads * kMultipleFastMaxCols;
+}
+int MultipleFastTiles(const Shape& s) {
+  const int rows = MultipleByNodes(s) ? NodeRows(s) : MultipleDims(s).rows;
+  return (s.sr * s.smu + rows - 1) / rows;
+}
+int MultipleFastSmem(const Shape& s) {
+  if (MultipleByNodes(s))
+    return NodeRows(s) * (kRaySamples * (int)sizeof(RaySample) + 4 * s.smus * 16);
+  const MultipleFastDims d = MultipleDims(s);
+  return d.rows * kRaySamples * (int)sizeof(RaySample) + 2 * d.group * d.rows * s.sw() * 16;
+}
+
 cudaError_t LaunchMultipleFast(const Instance* insts, WorkList wl, int tiles, int smem_bytes,
                                cudaStream_t st) {
   // smem_bytes: the largest MultipleFastSmem of the work list's instances.
-  k_multiple_fast<<<tiles, kMultipleFastThreads, (size_t)smem_bytes, st>>>(insts, wl);
+  const size_t bytes = (size_t)smem_bytes;
+  if (wl.kinds & 1) k_multiple_nodes<1><<<tiles, kMultipleFastThreads, bytes, st>>>(insts, wl);
+  if (wl.kinds & 2) k_multiple_nodes<2><<<tiles, kMultipleFastThreads, bytes, st>>>(insts, wl);
+  if (wl.kinds & 4) k_multiple_fast<<<tiles, kMultipleFastThreads, bytes, st>>>(insts, wl);
   return cudaGetLastError();
 }
 

@@ -43,7 +43,21 @@ struct WorkList {
   const int* inst;
   const int* start;
   int count;
+  int kinds;   // the instances' MultipleKind bits
 };
+
+// The multiple-scattering kernel of a LUT shape, a bit: 1, the mu_s columns of
+// a nu node in one register per lane (MU_S <= 32, where the 32 / MU_S nodes of
+// a warp fill 3/4 of its lanes); 2, in two (MU_S 33 to 64 and more than 256
+// columns in all); 4, lines in shared memory.  4 instances of 32 x 128 rows,
+// kernel 4 against the other, ms: MU_S x NU = 8 x 8 0.301 / 0.244, 32 x 8
+// 1.10 / 0.87, 11 x 8 (22 lanes) 0.439 / 0.461, 19 x 8 (19 lanes) 0.766 /
+// 0.844; 40 x 8 1.99 / 1.66, 64 x 8 2.40 / 1.66, 64 x 3 (192 columns, one per
+// thread of kernel 4) 0.839 / 1.062.
+ATMO_HD int MultipleKind(const Shape& s) {
+  if (s.smus <= 32) return 32 / s.smus * s.smus >= 24 ? 1 : 4;
+  return s.smus <= 64 && s.sw() > 256 ? 2 : 4;
+}
 
 #ifdef __CUDACC__
 // Finds the work-list entry holding `tile` (binary search over start[]).

@@ -288,6 +288,7 @@ extern "C" atmo_status atmo_precompute_noalloc(const atmo_atmosphere* atmosphere
     wl.inst = d_wl + 3 * i;
     wl.start = d_wl + 3 * i + 1;
     wl.count = 1;
+    wl.kinds = MultipleKind(s);
     e = LaunchPass(steps[i].pass, steps[i].order, steps[i].smem, d_in, wl, steps[i].tiles,
                    steps[i].path, st);
     if (e != cudaSuccess) return CudaFail(e, "kernel launch");

@@ -152,6 +152,7 @@ extern "C" atmo_status atmo_run_pass(const atmo_atmosphere* atmosphere,
     wl.inst = d_wl + 3 * i;
     wl.start = d_wl + 3 * i + 1;
     wl.count = 1;
+    wl.kinds = MultipleKind(s);
     return wl;
   };
   atmo_status result = ATMO_OK;

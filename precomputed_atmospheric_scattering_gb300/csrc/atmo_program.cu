@@ -305,6 +305,8 @@ atmo_status Program::Finalize() {
     w.inst = d_blob_ + o.first;
     w.start = d_blob_ + o.first + o.second;
     w.count = o.second;
+    w.kinds = 0;
+    for (int i = 0; i < o.second; ++i) w.kinds |= MultipleKind(slots[blob_[o.first + i]].s);
     wls_.push_back(w);
   }
   ATMO_CUDA_TRY(cudaMalloc(&d_slots_, slots.size() * sizeof(Instance)));

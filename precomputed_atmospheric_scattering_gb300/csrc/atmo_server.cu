@@ -471,8 +471,9 @@ bool atmo_server::LaunchRound() {
   size_t off = 0;
   for (const Group& g : groups) {
     const size_t n = g.members.size();
-    int t = 0, smem = 0;
+    int t = 0, smem = 0, kinds = 0;
     for (size_t i = 0; i < n; ++i) {
+      kinds |= MultipleKind(g.members[i]->s);
       h[off + i] = g.members[i]->index;
       h[off + n + i] = t;
       t += Tiles(g.pass, g.members[i]->s, g.path);
@@ -484,6 +485,7 @@ bool atmo_server::LaunchRound() {
     wl.inst = d_ring + ring_head + off;
     wl.start = d_ring + ring_head + off + n;
     wl.count = (int)n;
+    wl.kinds = kinds;
     launches.push_back(Launch{g.pass, g.order, t, smem, g.path, wl});
     off += 2 * n + 1;
   }
