@@ -43,7 +43,7 @@ struct WorkList {
   const int* inst;
   const int* start;
   int count;
-  int kinds;   // the instances' MultipleKind bits
+  int kinds;   // the instances' KernelKinds bits
 };
 
 // The multiple-scattering kernel of a LUT shape, a bit: 1, the mu_s columns of
@@ -58,6 +58,21 @@ ATMO_HD int MultipleKind(const Shape& s) {
   if (s.smus <= 32) return 32 / s.smus * s.smus >= 24 ? 1 : 4;
   return s.smus <= 64 && s.sw() > 256 ? 2 : 4;
 }
+
+// The scattering-density kernel of a LUT shape above order 2, a bit: arcs, 4
+// or 8 nu nodes per warp, or a table lookup per direction.  A warp of the arcs
+// is a long chain that needs blocks enough to fill the chip, and its work
+// grows with NU.  One instance, lookups / arcs, us: texels 57 k at NU 5 51 /
+// 43, 66 k at NU 4 51 / 39 and at NU 8 37 / 49, 131 k at NU 8 55 / 49, 262 k
+// at NU 16 104 / 102, 1 M at NU 8 301 / 182 (with 4 nodes per warp 219); 4 of
+// 2 M at NU 16 2258 / 1999.  Small LUTs take 4 nodes per warp: more warps.
+constexpr int kDensityArcs4 = 8, kDensityArcs8 = 16, kDensityLookups = 32;
+ATMO_HD int DensityKind(const Shape& s) {
+  const long long texels = s.s_texels();
+  if (s.snu > 16 || s.iw > 512 || texels < (s.snu <= 5 ? 49152 : 131072)) return kDensityLookups;
+  return s.snu <= 4 || texels < 262144 ? kDensityArcs4 : kDensityArcs8;
+}
+ATMO_HD int KernelKinds(const Shape& s) { return MultipleKind(s) | DensityKind(s); }
 
 #ifdef __CUDACC__
 // Finds the work-list entry holding `tile` (binary search over start[]).

@@ -24,7 +24,7 @@ cudaError_t LaunchIndirectIrradiance(const Instance* insts, WorkList wl, int til
 cudaError_t LaunchMultiplePlain(const Instance* insts, WorkList wl, int tiles,
                                 cudaStream_t st);
 // Fast path (atmo_fast.cu).
-int DensityFastTiles(const Shape& s);
+int DensityFastTiles(const Shape& s, int order);
 int DensityFastSmem(const Shape& s, const Consts& c, int order);
 cudaError_t PrepareDensityFast();
 bool DensityFastFits(const Shape& s);

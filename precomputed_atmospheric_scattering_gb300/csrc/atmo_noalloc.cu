@@ -224,7 +224,7 @@ extern "C" atmo_status atmo_precompute_noalloc(const atmo_atmosphere* atmosphere
   auto add = [&](Pass p, int order) {
     const atmo_path path = PassPath(p, s, ATMO_PATH_FAST);
     steps.push_back(
-        PlannedStep{p, order, Tiles(p, s, path), SharedBytes(p, s, consts, order, path), path});
+        PlannedStep{p, order, Tiles(p, s, path, order), SharedBytes(p, s, consts, order, path), path});
   };
   add(Pass::kTables, 0);
   add(Pass::kTransmittance, 0);
@@ -288,7 +288,7 @@ extern "C" atmo_status atmo_precompute_noalloc(const atmo_atmosphere* atmosphere
     wl.inst = d_wl + 3 * i;
     wl.start = d_wl + 3 * i + 1;
     wl.count = 1;
-    wl.kinds = MultipleKind(s);
+    wl.kinds = KernelKinds(s);
     e = LaunchPass(steps[i].pass, steps[i].order, steps[i].smem, d_in, wl, steps[i].tiles,
                    steps[i].path, st);
     if (e != cudaSuccess) return CudaFail(e, "kernel launch");

@@ -131,8 +131,8 @@ extern "C" atmo_status atmo_run_pass(const atmo_atmosphere* atmosphere,
 
   const atmo_path pp = PassPath(p, s, path);
   const int step_order = (int)order;
-  const int tiles[3] = {Tiles(Pass::kTables, s, path), Tiles(Pass::kDirect, s, path),
-                        Tiles(p, s, pp)};
+  const int tiles[3] = {Tiles(Pass::kTables, s, path, 0), Tiles(Pass::kDirect, s, path, 0),
+                        Tiles(p, s, pp, step_order)};
   struct {
     Instance in[2];
     int wl[9];
@@ -152,7 +152,7 @@ extern "C" atmo_status atmo_run_pass(const atmo_atmosphere* atmosphere,
     wl.inst = d_wl + 3 * i;
     wl.start = d_wl + 3 * i + 1;
     wl.count = 1;
-    wl.kinds = MultipleKind(s);
+    wl.kinds = KernelKinds(s);
     return wl;
   };
   atmo_status result = ATMO_OK;

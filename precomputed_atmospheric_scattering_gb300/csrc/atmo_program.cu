@@ -194,7 +194,7 @@ int SharedBytes(Pass pass, const Shape& s, const Consts& c, int order, atmo_path
   return 0;
 }
 
-int Tiles(Pass pass, const Shape& s, atmo_path path) {
+int Tiles(Pass pass, const Shape& s, atmo_path path, int order) {
   auto cdiv = [](long long a, long long b) { return (int)((a + b - 1) / b); };
   switch (pass) {
     case Pass::kTables: return TableTiles(s);
@@ -203,7 +203,7 @@ int Tiles(Pass pass, const Shape& s, atmo_path path) {
     case Pass::kSingle:
       return path == ATMO_PATH_FAST ? SingleFastTiles(s) : cdiv(s.s_texels(), kTexelThreads);
     case Pass::kDensity:
-      return path == ATMO_PATH_FAST ? DensityFastTiles(s) : cdiv(s.s_texels(), kTexelThreads);
+      return path == ATMO_PATH_FAST ? DensityFastTiles(s, order) : cdiv(s.s_texels(), kTexelThreads);
     case Pass::kIndirect: return cdiv(s.i_texels(), kIndirectTexelsPerTile);
     case Pass::kMultiple:
       return path == ATMO_PATH_FAST ? MultipleFastTiles(s) : cdiv(s.s_texels(), kTexelThreads);
@@ -244,7 +244,7 @@ int Program::AddWorkList(const std::vector<int>& members, Pass pass, int order, 
     if (!takes_part(m)) continue;
     inst.push_back(m);
     start.push_back(t);
-    t += Tiles(pass, slots[m].s, p);
+    t += Tiles(pass, slots[m].s, p, order);
     if (smem) {
       int b = SharedBytes(pass, slots[m].s, slots[m].c, order, p);
       *smem = b > *smem ? b : *smem;
@@ -306,7 +306,7 @@ atmo_status Program::Finalize() {
     w.start = d_blob_ + o.first + o.second;
     w.count = o.second;
     w.kinds = 0;
-    for (int i = 0; i < o.second; ++i) w.kinds |= MultipleKind(slots[blob_[o.first + i]].s);
+    for (int i = 0; i < o.second; ++i) w.kinds |= KernelKinds(slots[blob_[o.first + i]].s);
     wls_.push_back(w);
   }
   ATMO_CUDA_TRY(cudaMalloc(&d_slots_, slots.size() * sizeof(Instance)));

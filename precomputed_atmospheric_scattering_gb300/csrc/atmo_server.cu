@@ -473,10 +473,10 @@ bool atmo_server::LaunchRound() {
     const size_t n = g.members.size();
     int t = 0, smem = 0, kinds = 0;
     for (size_t i = 0; i < n; ++i) {
-      kinds |= MultipleKind(g.members[i]->s);
+      kinds |= KernelKinds(g.members[i]->s);
       h[off + i] = g.members[i]->index;
       h[off + n + i] = t;
-      t += Tiles(g.pass, g.members[i]->s, g.path);
+      t += Tiles(g.pass, g.members[i]->s, g.path, g.order);
       smem = std::max(smem, SharedBytes(g.pass, g.members[i]->s, h_inst[g.members[i]->index].c,
                                         g.order, g.path));
     }
