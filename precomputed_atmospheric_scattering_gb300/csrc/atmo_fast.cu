@@ -59,9 +59,10 @@ constexpr int kPairBytes = 48;
 // Three channels as a register pair (x, y) and a scalar (z) for the packed
 // FP32x2 instructions (per component the same IEEE operations as fmaf and
 // fadd, so the sums are bit-identical to the scalar ones).  Above order 2 the
-// density kernel is bound by instruction issue, and the packed FMAs and adds
-// of its lookups and sums save ~3% of its time.  At order 2 they do not pay:
-// its code stays scalar.
+// packed FMAs and adds of the lookups and sums save ~3% of the kernel's time.
+// At order 2 they do not pay, although they save 11% of the instructions: a
+// packed FMA holds the FMA pipe for two slots or more (9.8 ms per launch
+// against 9.0), only the packed products are free.
 struct P3 {
   float2 xy;
   float z;
@@ -210,8 +211,12 @@ __device__ __forceinline__ void EvalPair(float s, float t, uint32_t row_adj, F3*
   *ray = F3{fmaf(s, p.w, p.x), fmaf(s, q.x, p.y), fmaf(s, q.y, p.z)};
   *mie = F3{fmaf(s, r.y, q.z), fmaf(s, r.z, q.w), fmaf(s, r.w, r.x)};
 }
-__host__ __device__ constexpr uint32_t RowAdjust(uint32_t base, int stride) {
-  return base - kRoundMagicBits * (uint32_t)stride;
+// magic: kRoundMagic, as a run-time value.  With the constant in sight the
+// compiler merges it with the loads' offsets into terms too large for a load's
+// immediate and adds each to the address: one more instruction per load (3 of
+// 34 per sample at order 2, whose 16-instance launch took 9.08 ms, now 8.47).
+__device__ __forceinline__ uint32_t RowAdjust(uint32_t base, int stride, float magic) {
+  return base - (uint32_t)__float_as_int(magic) * (uint32_t)stride;
 }
 
 // Ground rows above order 2.  On a theta row whose directions hit the ground
@@ -295,6 +300,24 @@ struct DensityTask {
   V sum[kN];              // sums of L (a_R P_R(nu2) + a_M P_M(nu2)) dw
 };
 
+// Ground rows at order 2: the irradiance seen along a theta row is linear in
+// s on nearly every row (the directions reach one irradiance interval), or has
+// one kink; then it needs no lookup, and its sum over the two sides of a phi
+// pair no more than their s: base + slope (s0 + s1) + bend (max(s0 - kink, 0)
+// + max(s1 - kink, 0)) (base twice the line's).  More intervals: lookups.
+// The lookups were 18% of the kernel's shared-memory wavefronts and 6 of 38
+// instructions per sample; without them the 16-instance launch at the
+// reference's shape takes 9.08 ms instead of 10.31.
+enum GroundForm { kNoGround, kGroundLine, kGroundKink, kGroundLookup };
+struct __align__(16) GroundRow {
+  F3 base;
+  int form;
+  F3 slope;
+  float kink;
+  F3 bend;
+  float pad;
+};
+
 // The 32 phi samples of theta row l for the texels of one task.  Everything
 // is in the unit coordinate s = 1/2 + k1 nu1 (k1 = (NU - 1) / (2 NU)) of the
 // staged rows: A is s's part 1/2 + k1 mu_s cos(theta_l), hs = k1 sin(theta_l)
@@ -305,24 +328,34 @@ struct DensityTask {
 // scattering coefficients at the texel times the phase constants and dw.
 // kMerged (ground rows above order 2): the row's merged table (MergeRow)
 // replaces the sky and ground lookups.
-template <bool kOrder2, bool kGround, bool kMerged = false>
+template <bool kOrder2, int kForm, bool kMerged = false>
 __device__ __forceinline__ void DensityThetaRow(DensityTask<kOrder2>& task,
                                                 const Consts& c, float A, float hs, float B,
                                                 float oxs, F3 war, F3 wam, float fnu,
-                                                float inv_k1, uint32_t row_adj, F3 tg,
+                                                float inv_k1, float magic, uint32_t row_adj, F3 tg,
                                                 float g_scale, float g_off, float fiw,
                                                 uint32_t ir_adj, uint32_t jstride = 0,
-                                                uint32_t madj = 0) {
+                                                uint32_t madj = 0,
+                                                const GroundRow* ground = nullptr) {
+  constexpr bool kGround = kForm == kGroundLookup;
   static_assert(!kMerged || (kGround && !kOrder2), "merged tables: ground rows above order 2");
-  using V = typename DensityTask<kOrder2>::V;
+  [[maybe_unused]] F3 g_base = f3(0.0f), g_slope = f3(0.0f), g_bend = f3(0.0f);
+  [[maybe_unused]] float g_kink = 0.0f;
+  if constexpr (kForm == kGroundLine || kForm == kGroundKink) {
+    g_base = ground->base;
+    g_slope = ground->slope;
+    if constexpr (kForm == kGroundKink) {
+      g_bend = ground->bend;
+      g_kink = ground->kink;
+    }
+  }
   constexpr int kDensityTexelsPerTask = DensityTexelsPerTask<kOrder2>();
-  const float m2g = c.m2g, g2p1 = c.g2p1;
+  [[maybe_unused]] const float m2g = c.m2g, g2p1 = c.g2p1;
   // phi and 2 pi - phi share cos(phi), hence nu2 and the phase functions of
   // the outgoing direction; nu1 differs by the sign of sy sin(phi).  Unrolled
-  // 4 times above order 2, not at order 2 (measured: -1.7% and -1.2%
-  // against 2; with the packed arithmetic, 2 and 8 are 2% and 5% slower
-  // than 4 above order 2).
-#pragma unroll(kOrder2 ? 1 : 4)
+  // 4 times above order 2, twice at order 2 (8.27 ms per 16-instance launch
+  // against 8.47; 4 times overflows the instruction cache: 9.38).
+#pragma unroll(kOrder2 ? 2 : 4)
   for (int m = 0; m < kDensityPhiSamples / 2; ++m) {
     const float2 cs = c_density_phi[m];
     // Phase functions at nu2 (functions.glsl:739-747, :1245-1254), folded
@@ -332,62 +365,71 @@ __device__ __forceinline__ void DensityThetaRow(DensityTask<kOrder2>& task,
     // 1 + g^2 - 2 g nu2 >= (1 - g)^2: zero or normal for |g| < 1.
     const float rs = RsqrtFtz(fmaf(m2g, nu2, g2p1));
     const F3 wf = fma3(wam, q2 * (rs * rs * rs), war * q2);
-    const P3 w = ToP3(wf);
     const float hc = cs.x * hs, hn = cs.y * hs;
 #pragma unroll
     for (int q = 0; q < kDensityTexelsPerTask; ++q) {
       // The unit coordinate of nu1: bu +- sy sin(theta) sin(phi) / 2.
       const float bu = fmaf(task.sx[q], hc, A);
-      // Ls is seeded with the first side's radiance (an explicit 0 + x
-      // would cost an add per channel: IEEE keeps it).
-      V Ls;
+      const float2 u2 =
+          make_float2(FmaSat(hn, task.sy[q], bu), FmaSat(-hn, task.sy[q], bu));
+      if constexpr (kOrder2) {
+        // Single scattering with its phase functions at nu1 (:998-1004):
+        // (1 + nu1^2) (R 3/(16 pi) + M k_M / (1 + g^2 - 2 g nu1)^(3/2)),
+        // with the constant factors staged into the tables.
+        const float n0 = fmaf(u2.x, inv_k1, -0.5f * inv_k1);
+        const float n1 = fmaf(u2.y, inv_k1, -0.5f * inv_k1);
+        const float2 r1 = make_float2(RsqrtFtz(fmaf(m2g, n0, g2p1)), RsqrtFtz(fmaf(m2g, n1, g2p1)));
+        const float2 r3 = __fmul2_rn(__fmul2_rn(r1, r1), r1);
+        F3 Ls;
+        if constexpr (kForm == kGroundLine || kForm == kGroundKink) {
+          Ls = fma3(g_slope, u2.x + u2.y, g_base);
+          if constexpr (kForm == kGroundKink)
+            Ls = fma3(g_bend, fmaxf(u2.x - g_kink, 0.0f) + fmaxf(u2.y - g_kink, 0.0f), Ls);
+        }
 #pragma unroll
-      for (int side = 0; side < 2; ++side) {
-        const float u = FmaSat(side == 0 ? hn : -hn, task.sy[q], bu);
-        const float t = fmaf(u, fnu, kRoundMagic);
-        if constexpr (kMerged) {
-          // Entry (i, j) of the merged table: one line in s for sky + ground.
-          const float x = FmaSat(u, g_scale, g_off);
-          const uint32_t a = (uint32_t)__float_as_int(t) * jstride +
-                             (uint32_t)__float_as_int(fmaf(x, fiw, kRoundMagic)) *
-                                 (uint32_t)kNodeBytes +
-                             madj;
-          const P3 L = PackedLine(u, a);
-          Ls = side == 0 ? L : Add(Ls, L);
-          continue;
-        }
-        if constexpr (kOrder2) {
+        for (int side = 0; side < 2; ++side) {
+          const float u = side == 0 ? u2.x : u2.y, nu1 = side == 0 ? n0 : n1;
           F3 L, M;
-          EvalPair(u, t, row_adj, &L, &M);
-          // Single scattering with its phase functions at nu1 (:998-1004):
-          // (1 + nu1^2) (R 3/(16 pi) + M k_M / (1 + g^2 - 2 g nu1)^(3/2)),
-          // with the constant factors staged into the tables.
-          const float nu1 = fmaf(u, inv_k1, -0.5f * inv_k1);
-          const float r1 = RsqrtFtz(fmaf(m2g, nu1, g2p1));
-          const F3 L1 = fma3(M, r1 * r1 * r1, L);
+          EvalPair(u, fmaf(u, fnu, magic), row_adj, &L, &M);
+          const F3 L1 = fma3(M, side == 0 ? r3.x : r3.y, L);
           const float q1 = fmaf(nu1, nu1, 1.0f);
-          Ls = side == 0 ? L1 * q1 : fma3(L1, q1, Ls);
-        } else {
-          const P3 L = EvalNodesPacked(u, t, row_adj);
-          Ls = side == 0 ? L : Add(Ls, L);
-        }
-        if (kGround) {
-          // Ground bounce: the ground point is at radius Rb, so the cosine
-          // of its normal with the sun is (r mu_s + dist nu1) / Rb; the
-          // irradiance lookup at r = Rb reads row 0 of the LUT.
-          const float x = FmaSat(u, g_scale, g_off);
-          const float xt = fmaf(x, fiw, kRoundMagic);
-          if constexpr (kOrder2) {
-            Ls = fma3(tg, EvalNodes<kNodeBytes, 0>(x, xt, ir_adj), Ls);
-          } else {
-            Ls = Fma(ToP3(tg), EvalNodesPacked(x, xt, ir_adj), Ls);
+          Ls = side == 0 && (kForm == kNoGround || kGround) ? L1 * q1 : fma3(L1, q1, Ls);
+          if (kGround) {
+            // Ground bounce: the ground point is at radius Rb, so the cosine
+            // of its normal with the sun is (r mu_s + dist nu1) / Rb; the
+            // irradiance lookup at r = Rb reads row 0 of the LUT.
+            const float x = FmaSat(u, g_scale, g_off);
+            Ls = fma3(tg, EvalNodes<kNodeBytes, 0>(x, fmaf(x, fiw, magic), ir_adj), Ls);
           }
         }
-      }
-      if constexpr (kOrder2) {
         task.sum[q] = fma3(Ls, wf, task.sum[q]);
       } else {
-        task.sum[q] = Fma(Ls, w, task.sum[q]);
+        // Ls is seeded with the first side's radiance (an explicit 0 + x
+        // would cost an add per channel: IEEE keeps it).
+        P3 Ls;
+#pragma unroll
+        for (int side = 0; side < 2; ++side) {
+          const float u = side == 0 ? u2.x : u2.y, t = fmaf(u, fnu, magic);
+          if constexpr (kMerged) {
+            // Entry (i, j) of the merged table: one line in s for sky + ground.
+            const float x = FmaSat(u, g_scale, g_off);
+            const uint32_t a = (uint32_t)__float_as_int(t) * jstride +
+                               (uint32_t)__float_as_int(fmaf(x, fiw, magic)) *
+                                   (uint32_t)kNodeBytes +
+                               madj;
+            const P3 L = PackedLine(u, a);
+            Ls = side == 0 ? L : Add(Ls, L);
+            continue;
+          }
+          const P3 L = EvalNodesPacked(u, t, row_adj);
+          Ls = side == 0 ? L : Add(Ls, L);
+          if (kGround) {
+            // The ground bounce, as at order 2.
+            const float x = FmaSat(u, g_scale, g_off);
+            Ls = Fma(ToP3(tg), EvalNodesPacked(x, fmaf(x, fiw, magic), ir_adj), Ls);
+          }
+        }
+        task.sum[q] = Fma(Ls, ToP3(wf), task.sum[q]);
       }
     }
   }
@@ -395,7 +437,8 @@ __device__ __forceinline__ void DensityThetaRow(DensityTask<kOrder2>& task,
 
 template <bool kOrder2>
 __global__ void __launch_bounds__(kDensityFastThreads)
-k_density_fast(const Instance* __restrict__ insts, WorkList wl, int order, int smem_bytes) {
+k_density_fast(const Instance* __restrict__ insts, WorkList wl, int order, int smem_bytes,
+               float magic) {
   extern __shared__ float4 smem[];
   constexpr int kSpecies = kOrder2 ? 2 : 1;
   constexpr int kStride = kOrder2 ? kPairBytes : kNodeBytes;
@@ -534,9 +577,47 @@ k_density_fast(const Instance* __restrict__ insts, WorkList wl, int order, int s
   }
   __syncthreads();
 
+  // Order 2: the ground rows' forms, in place of the node values.
+  GroundRow* grounds = reinterpret_cast<GroundRow*>(V);
+  if (kOrder2 && threadIdx.x < kDensityThetaSamples) {
+    const DensityRow dr = drows[threadIdx.x];
+    GroundRow g;
+    g.base = g.slope = g.bend = f3(0.0f);
+    g.kink = g.pad = 0.0f;
+    g.form = dr.ground ? kGroundLookup : kNoGround;
+    if (dr.ground) {
+      // The irradiance entries reached from s = 1/2 + k1 (mu_s cos(theta) -+
+      // sin_s sin(theta)).
+      const float gs = kg * dr.dist_ground * inv_rb * inv_k1;
+      const float go = fmaf(-0.5f, gs, fmaf(in.tab.rows[k * s.smu].r * cc.mu_s * inv_rb, kg, 0.5f));
+      const float mid = fmaf(cc.mu_s * dr.cos_t, k1, 0.5f), half = k1 * dr.sin_t * cc.sin_s;
+      const int j0 = __float_as_int(fmaf(FmaSat(mid - half, gs, go), fiw, kRoundMagic)) -
+                     (int)kRoundMagicBits;
+      const int j1 = __float_as_int(fmaf(FmaSat(mid + half, gs, go), fiw, kRoundMagic)) -
+                     (int)kRoundMagicBits;
+      if (j1 <= j0 + 1) {
+        const float4* e0 = G + j0 * (kNodeBytes / 16);
+        const float4* e1 = G + j1 * (kNodeBytes / 16);
+        const F3 tg = f3(dr.t_ground);
+        const F3 a{e0[0].x, e0[0].y, e0[0].z}, b{e0[0].w, e0[1].x, e0[1].y};
+        g.base = tg * fma3(b, go, a) * 2.0f;
+        g.slope = tg * b * gs;
+        g.form = kGroundLine;
+        if (j1 > j0) {
+          // Entries j0 and j0 + 1 meet at node j0: (j0 + 1/2) / IW.
+          g.form = kGroundKink;
+          g.bend = tg * (F3{e1[0].w, e1[1].x, e1[1].y} - b) * gs;
+          g.kink = ((float(j0) + 0.5f) / fiw - go) / gs;
+        }
+      }
+    }
+    grounds[threadIdx.x] = g;
+  }
+  if (kOrder2) __syncthreads();
+
   const float dtdp = (kPiF / 16.0f) * (kPiF / 16.0f);
   const uint32_t e_base = (uint32_t)__cvta_generic_to_shared(E);
-  const uint32_t ir_adj = RowAdjust((uint32_t)__cvta_generic_to_shared(G), kNodeBytes);
+  const uint32_t ir_adj = RowAdjust((uint32_t)__cvta_generic_to_shared(G), kNodeBytes, magic);
   const int per_row = (NU + kDensityTexelsPerTask - 1) / kDensityTexelsPerTask;
   const int tasks = s.smu * per_row;
   for (int ti = threadIdx.x; ti < tasks; ti += blockDim.x) {
@@ -565,30 +646,43 @@ k_density_fast(const Instance* __restrict__ insts, WorkList wl, int order, int s
       const float A = fmaf(cc.mu_s * dr.cos_t, k1, 0.5f);
       const float hs = k1 * dr.sin_t;
       const uint32_t row_adj =
-          RowAdjust(e_base + (uint32_t)(l * row_entries * kStride), kStride);
-      if (dr.ground) {
-        if constexpr (kOrder2) {
+          RowAdjust(e_base + (uint32_t)(l * row_entries * kStride), kStride, magic);
+      if constexpr (kOrder2) {
+        const GroundRow* g = grounds + l;
+        if (g->form == kGroundLine) {
+          DensityThetaRow<kOrder2, kGroundLine>(task, c, A, hs, B, oxs, a_r * dw, a_m * dw, fnu,
+                                                inv_k1, magic, row_adj, f3(0.0f), 0.0f, 0.0f, fiw, ir_adj,
+                                                0, 0, g);
+        } else if (g->form == kGroundKink) {
+          DensityThetaRow<kOrder2, kGroundKink>(task, c, A, hs, B, oxs, a_r * dw, a_m * dw, fnu,
+                                                inv_k1, magic, row_adj, f3(0.0f), 0.0f, 0.0f, fiw, ir_adj,
+                                                0, 0, g);
+        } else if (g->form == kGroundLookup) {
           // The ground point's irradiance coordinate from s = 1/2 + k1 nu1:
           // w0 + kg dist (s - 1/2) / (k1 Rb).
           const float gs = kg * dr.dist_ground * inv_rb * inv_k1;
           const float go = fmaf(-0.5f, gs, w0);
-          DensityThetaRow<kOrder2, true>(task, c, A, hs, B, oxs, a_r * dw, a_m * dw, fnu,
-                                         inv_k1, row_adj, f3(dr.t_ground), gs, go, fiw, ir_adj);
+          DensityThetaRow<kOrder2, kGroundLookup>(task, c, A, hs, B, oxs, a_r * dw, a_m * dw, fnu,
+                                                  inv_k1, magic, row_adj, f3(dr.t_ground), gs, go, fiw,
+                                                  ir_adj);
         } else {
-          const MergeRow mr = meta[l];
-          if (mr.jstride != 0) {
-            DensityThetaRow<kOrder2, true, true>(task, c, A, hs, B, oxs, a_r * dw, a_m * dw,
-                                                 fnu, inv_k1, row_adj, f3(0.0f), mr.gs, mr.go,
-                                                 fiw, ir_adj, mr.jstride, mr.adj);
-          } else {
-            DensityThetaRow<kOrder2, true>(task, c, A, hs, B, oxs, a_r * dw, a_m * dw, fnu,
-                                           inv_k1, row_adj, f3(dr.t_ground), mr.gs, mr.go, fiw,
-                                           ir_adj);
-          }
+          DensityThetaRow<kOrder2, kNoGround>(task, c, A, hs, B, oxs, a_r * dw, a_m * dw, fnu,
+                                              inv_k1, magic, row_adj, f3(0.0f), 0.0f, 0.0f, fiw, ir_adj);
+        }
+      } else if (dr.ground) {
+        const MergeRow mr = meta[l];
+        if (mr.jstride != 0) {
+          DensityThetaRow<kOrder2, kGroundLookup, true>(
+              task, c, A, hs, B, oxs, a_r * dw, a_m * dw, fnu, inv_k1, magic, row_adj, f3(0.0f), mr.gs,
+              mr.go, fiw, ir_adj, mr.jstride, mr.adj);
+        } else {
+          DensityThetaRow<kOrder2, kGroundLookup>(task, c, A, hs, B, oxs, a_r * dw, a_m * dw, fnu,
+                                                  inv_k1, magic, row_adj, f3(dr.t_ground), mr.gs, mr.go,
+                                                  fiw, ir_adj);
         }
       } else {
-        DensityThetaRow<kOrder2, false>(task, c, A, hs, B, oxs, a_r * dw, a_m * dw, fnu, inv_k1,
-                                        row_adj, f3(0.0f), 0.0f, 0.0f, fiw, ir_adj);
+        DensityThetaRow<kOrder2, kNoGround>(task, c, A, hs, B, oxs, a_r * dw, a_m * dw, fnu, inv_k1,
+                                            magic, row_adj, f3(0.0f), 0.0f, 0.0f, fiw, ir_adj);
       }
     }
 #pragma unroll
@@ -973,7 +1067,8 @@ cudaError_t LaunchDensityFast(const Instance* insts, WorkList wl, int tiles, int
   // smem_bytes: the largest DensityFastSmem of the work list's instances.
   const size_t bytes = (size_t)smem_bytes;
   if (order == 2) {
-    k_density_fast<true><<<tiles, kDensityFastThreads, bytes, st>>>(insts, wl, order, smem_bytes);
+    k_density_fast<true><<<tiles, kDensityFastThreads, bytes, st>>>(insts, wl, order, smem_bytes,
+                                                                      kRoundMagic);
   } else {
     if (smem_bytes > 48 * 1024) {
       const cudaError_t e = PrepareDensityFast();
@@ -987,7 +1082,7 @@ cudaError_t LaunchDensityFast(const Instance* insts, WorkList wl, int tiles, int
     if (wl.kinds & kDensityLookups) {
       const int fast_bytes = std::min(smem_bytes, kDensityMaxSmem);
       k_density_fast<false><<<tiles, kDensityFastThreads, (size_t)fast_bytes, st>>>(
-          insts, wl, order, fast_bytes);
+          insts, wl, order, fast_bytes, kRoundMagic);
     }
   }
   return cudaGetLastError();
