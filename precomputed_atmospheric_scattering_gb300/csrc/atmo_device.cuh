@@ -82,13 +82,39 @@ ATMO_HD F3 ratio3(F3 a, F3 b) {
 ATMO_HD F3 exp3(F3 a) { return F3{expf(a.x), expf(a.y), expf(a.z)}; }
 ATMO_HD float4 to4(F3 a, float w) { return make_float4(a.x, a.y, a.z, w); }
 
+// Quotient and square root of the geometry below.  A translation unit that
+// defines ATMO_FLUSHED_GEOMETRY gets the approximate forms that flush
+// subnormal operands to zero (PTX .approx.ftz, <= 2 ulp like the .approx forms
+// of --prec-div=false and --prec-sqrt=false, but without their range check and
+// rescaling: 2 instructions for 6): lengths, cosines and their quotients, where
+// a subnormal stands for zero.  Transmittances and radiances keep div_approx
+// and the division operator.
+ATMO_HD float quot(float a, float b) {
+#if defined(__CUDA_ARCH__) && defined(ATMO_FLUSHED_GEOMETRY)
+  float y;
+  asm("div.approx.ftz.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b));
+  return y;
+#else
+  return a / b;
+#endif
+}
+ATMO_HD float root(float x) {
+#if defined(__CUDA_ARCH__) && defined(ATMO_FLUSHED_GEOMETRY)
+  float y;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+#else
+  return sqrtf(x);
+#endif
+}
+
 ATMO_HD float clampf(float x, float lo, float hi) { return fminf(fmaxf(x, lo), hi); }
 // GLSL smoothstep; for the degenerate e0 == e1 (a point sun) it returns 0 at
 // x <= e0 and 1 above.
 ATMO_HD float smoothstepf(float e0, float e1, float x) {
   if (x <= e0) return 0.0f;
   if (x >= e1) return 1.0f;
-  float t = (x - e0) / (e1 - e0);
+  float t = quot(x - e0, e1 - e0);
   return t * t * (3.0f - 2.0f * t);
 }
 
@@ -163,9 +189,9 @@ struct RadialPoint {
 ATMO_HD RadialPoint PointFromRho2(const Consts& c, float rho2) {
   rho2 = clampf(rho2, 0.0f, c.H * c.H);
   RadialPoint p;
-  p.rho = sqrtf(rho2);
-  p.r = sqrtf(rho2 + c.Rb * c.Rb);
-  p.h = rho2 / (p.r + c.Rb);
+  p.rho = root(rho2);
+  p.r = root(rho2 + c.Rb * c.Rb);
+  p.h = quot(rho2, p.r + c.Rb);
   return p;
 }
 // Point at distance d along the ray (rho, r*mu): rho_d^2 = d^2 + 2 r mu d + rho^2.
@@ -180,8 +206,8 @@ ATMO_HD RadialPoint PointAlongRay(const Consts& c, float rho, float rmu, float d
 // -r mu + sqrt(H^2 - rho^2 + (r mu)^2), in its cancellation-free form.
 ATMO_HD float DistanceToTop(const Consts& c, float rho, float rmu) {
   float hm = (c.H - rho) * (c.H + rho);
-  float sq = sqrtf(fmaxf(fmaf(rmu, rmu, hm), 0.0f));
-  return rmu > 0.0f ? hm / (rmu + sq) : sq - rmu;
+  float sq = root(fmaxf(fmaf(rmu, rmu, hm), 0.0f));
+  return rmu > 0.0f ? quot(hm, rmu + sq) : sq - rmu;
 }
 
 // GL LINEAR + CLAMP_TO_EDGE bilinear fetch of RGB from a float4 2D texture.
@@ -228,12 +254,12 @@ struct TCoords {
 ATMO_HD TCoords TransmittanceCoords(const Consts& c, const Shape& s, float rho, float r,
                                     float rmu, float delta) {
   const float a = -rmu;
-  float sq = sqrtf(fmaxf(c.H * c.H - delta, 0.0f));
-  float rho_minus_a = a > 0.0f ? (rho + a > 0.0f ? delta / (rho + a) : 0.0f) : rho - a;
-  float dmax_minus_d = rho_minus_a + delta / (c.H + sq);
-  float d_min = (c.H - rho) * (c.H + rho) / (c.Rt + r);
+  float sq = root(fmaxf(c.H * c.H - delta, 0.0f));
+  float rho_minus_a = a > 0.0f ? (rho + a > 0.0f ? quot(delta, rho + a) : 0.0f) : rho - a;
+  float dmax_minus_d = rho_minus_a + quot(delta, c.H + sq);
+  float d_min = quot((c.H - rho) * (c.H + rho), c.Rt + r);
   float d_max = rho + c.H;
-  float omx = clampf(dmax_minus_d / (d_max - d_min), 0.0f, 1.0f);
+  float omx = clampf(quot(dmax_minus_d, d_max - d_min), 0.0f, 1.0f);
   // Texel coordinate X = x_mu (W - 1) = (W - 1) - Xc, fetched from the two
   // columns below W - 1 - floor(Xc) with weights computed from Xc itself.
   const int W = s.tw, Hh = s.th;
@@ -244,7 +270,7 @@ ATMO_HD TCoords TransmittanceCoords(const Consts& c, const Shape& s, float rho, 
   int i_lo = i_hi - 1;
   i_hi = i_hi < 0 ? 0 : i_hi;
   i_lo = i_lo < 0 ? 0 : i_lo;
-  float Y = rho / c.H * float(Hh - 1);
+  float Y = quot(rho, c.H) * float(Hh - 1);
   float fy = floorf(Y);
   float b = Y - fy;
   int j0 = (int)fy, j1 = j0 + 1;
@@ -299,7 +325,10 @@ ATMO_HD float MinTau(float a, float wa, float b, float wb, float c, float wc, fl
   if (wd > 0.0f) m = fminf(m, d);
   return m;
 }
-ATMO_HD TExp FetchTau(const float4* __restrict__ Tau, const TCoords& t) {
+#ifndef ATMO_RARE   // a translation unit may keep this seldom taken code out of line
+#define ATMO_RARE ATMO_HD
+#endif
+ATMO_RARE TExp FetchTau(const float4* __restrict__ Tau, const TCoords t) {
   float4 a = LoadTexel(Tau, t.i00), b = LoadTexel(Tau, t.i10);
   float4 c = LoadTexel(Tau, t.i01), d = LoadTexel(Tau, t.i11);
   TExp r;
@@ -374,9 +403,9 @@ ATMO_HD F3 SegmentTransmittance(const Consts& c, const Shape& s, const float4* T
 ATMO_HD F3 TransmittanceToSun(const Consts& c, const Shape& s, const float4* T,
                               const RadialPoint& p, float rmu_s) {
   rmu_s = clampf(rmu_s, -p.r, p.r);
-  float sin_theta_h = c.Rb / p.r;
+  float sin_theta_h = quot(c.Rb, p.r);
   // mu_s - cos(theta_h) with cos(theta_h) = -rho / r.
-  float x = (rmu_s + p.rho) / p.r;
+  float x = quot(rmu_s + p.rho, p.r);
   float e = sin_theta_h * c.alpha_s;
   return TransmittanceToTop(c, s, T, p.rho, p.r, rmu_s) * smoothstepf(-e, e, x);
 }
@@ -387,11 +416,11 @@ ATMO_HD F3 TransmittanceToSun(const Consts& c, const Shape& s, const float4* T,
 ATMO_HD float UMuSFromMuS(const Consts& c, const Shape& s, float mu_s) {
   // d = DistanceToTopAtmosphereBoundary(Rb, mu_s), cancellation-free.
   float rmus = c.Rb * mu_s;
-  float sq = sqrtf(fmaf(rmus, rmus, c.H * c.H));
-  float d = rmus > 0.0f ? (c.H * c.H) / (rmus + sq) : sq - rmus;
+  float sq = root(fmaf(rmus, rmus, c.H * c.H));
+  float d = rmus > 0.0f ? quot(c.H * c.H, rmus + sq) : sq - rmus;
   float d_min = c.Rt - c.Rb, d_max = c.H;
-  float a = (d - d_min) / (d_max - d_min);
-  return TexCoord(s, kMapSMUS, fmaxf(1.0f - a / c.mus_A, 0.0f) / (1.0f + a));
+  float a = quot(d - d_min, d_max - d_min);
+  return TexCoord(s, kMapSMUS, quot(fmaxf(1.0f - quot(a, c.mus_A), 0.0f), 1.0f + a));
 }
 
 // u_mu when the distance to the ray's boundary is known (d_ray).
@@ -399,12 +428,12 @@ ATMO_HD float UMuFromDistance(const Consts& c, const Shape& s, const RadialPoint
                               float d_ray, bool ground) {
   if (ground) {
     float d_min = p.h, d_max = p.rho;
-    float x = d_max == d_min ? 0.0f : clampf((d_ray - d_min) / (d_max - d_min), 0.0f, 1.0f);
+    float x = d_max == d_min ? 0.0f : clampf(quot(d_ray - d_min, d_max - d_min), 0.0f, 1.0f);
     return 0.5f - 0.5f * TexCoord(s, kMapSMU2, x);
   }
-  float d_min = (c.H - p.rho) * (c.H + p.rho) / (c.Rt + p.r);
+  float d_min = quot((c.H - p.rho) * (c.H + p.rho), c.Rt + p.r);
   float d_max = p.rho + c.H;
-  float x = clampf((d_ray - d_min) / (d_max - d_min), 0.0f, 1.0f);
+  float x = clampf(quot(d_ray - d_min, d_max - d_min), 0.0f, 1.0f);
   return 0.5f + 0.5f * TexCoord(s, kMapSMU2, x);
 }
 
@@ -415,8 +444,8 @@ ATMO_HD float UMuFromRMu(const Consts& c, const Shape& s, const RadialPoint& p, 
   if (ground) {
     // -r mu - sqrt((r mu)^2 - rho^2) = rho^2 / (-r mu + sqrt(...)).
     float disc = fmaxf((rmu - p.rho) * (rmu + p.rho), 0.0f);
-    float den = sqrtf(disc) - rmu;
-    d = den > 0.0f ? p.rho * p.rho / den : 0.0f;
+    float den = root(disc) - rmu;
+    d = den > 0.0f ? quot(p.rho * p.rho, den) : 0.0f;
   } else {
     d = DistanceToTop(c, p.rho, rmu);
   }
@@ -509,7 +538,7 @@ ATMO_HD float MiePhase(const Consts& c, float nu) {
 // Irradiance LUT (functions.glsl:1524-1533, :1595-1601).
 // ---------------------------------------------------------------------------
 ATMO_HD F3 Irradiance(const Consts& c, const Shape& s, const float4* I, float h, float mu_s) {
-  float x_r = h / (c.Rt - c.Rb);
+  float x_r = quot(h, c.Rt - c.Rb);
   float x_mu_s = mu_s * 0.5f + 0.5f;
   return Bilinear(I, s.iw, s.ih, TexCoord(s, kMapIW, x_mu_s), TexCoord(s, kMapIH, x_r));
 }

@@ -22,6 +22,7 @@ struct RenderLuts {
   const float4* M;      // single Mie (nullptr when combined)
   const float4* I;      // irradiance
   int combined;
+  float ray_over_mie, mie_over_ray[3];   // quotients of the scattering coefficients
   float sky_k[3];       // SKY_SPECTRAL_RADIANCE_TO_LUMINANCE
   float sun_k[3];       // SUN_SPECTRAL_RADIANCE_TO_LUMINANCE
 };
@@ -75,6 +76,10 @@ inline RenderLuts LutsOf(const Instance& in) {
   r.M = in.M;
   r.I = in.I;
   r.combined = in.combined;
+  r.ray_over_mie = in.c.rayleigh.x / in.c.mie_sca.x;
+  r.mie_over_ray[0] = in.c.mie_sca.x / in.c.rayleigh.x;
+  r.mie_over_ray[1] = in.c.mie_sca.y / in.c.rayleigh.y;
+  r.mie_over_ray[2] = in.c.mie_sca.z / in.c.rayleigh.z;
   for (int i = 0; i < 3; ++i) r.sky_k[i] = r.sun_k[i] = 1.0f;
   return r;
 }
