@@ -135,6 +135,18 @@ __device__ __forceinline__ float4 LoadShared4(uint32_t addr) {
   return v;
 }
 template <int kOffset>
+__device__ __forceinline__ F3 LoadShared3(uint32_t addr) {
+#ifdef ATMO_DEVICE_CHECKS
+  addr = CheckedShared(addr + kOffset, 12) - kOffset;
+#endif
+  F3 v;
+  asm volatile("ld.shared.f32 %0, [%3+%4];\n\tld.shared.f32 %1, [%3+%5];\n\t"
+               "ld.shared.f32 %2, [%3+%6];"
+               : "=&f"(v.x), "=&f"(v.y), "=&f"(v.z)
+               : "r"(addr), "n"(kOffset), "n"(kOffset + 4), "n"(kOffset + 8));
+  return v;
+}
+template <int kOffset>
 __device__ __forceinline__ float2 LoadShared2(uint32_t addr) {
 #ifdef ATMO_DEVICE_CHECKS
   addr = CheckedShared(addr + kOffset, 8) - kOffset;
@@ -1766,39 +1778,60 @@ cudaError_t LaunchMultipleFast(const Instance* insts, WorkList wl, int tiles, in
 // (rho, r): a fixed pair of transmittance LUT rows.  Per sample the block
 // interpolates those two rows into a line of W_T columns in shared memory; a
 // texel computes the x_mu of its sun direction and reads 2 line entries.
+//
+// Bound by the L1 data pipe (91% busy before the following, 37 wavefronts per
+// warp and sample): the lines' rows, the sample's constants and the taps.  So
+// an entry is three floats (a tap is three conflict-free 4-byte loads, where
+// 16-byte loads of scattered entries conflict), neighbouring lanes hold the nu
+// nodes of one mu_s column (whose taps start at one entry and drift apart
+// along the ray, and whose samples are in the planet's shadow together: a
+// shadowed sample reads nothing), a thread keeps its line columns of the last
+// two rows across samples, and two texel columns of a thread share a sample's
+// loads.  Per 16-instance launch at the reference's shape 3.55 -> 2.91 ms, one
+// high-resolution instance 2.74 -> 2.68 ms, one of half size 57 -> 47 us.
 // ---------------------------------------------------------------------------
 constexpr int kSingleSamples = kSingleScatteringSamples + 1;
+constexpr int kSingleThreads = 128;   // of a block of a shape of up to 256 columns
 
 struct __align__(16) SunSample {
-  int t0, t1;                // element offsets of the transmittance LUT rows j0, j1
-  float b;                   // weight of row j1
-  float rho, r, inv_r;       // the sample's rho, r and 1 / r
-  float inv_2e;              // 1 / (2 sin(theta_h) alpha_s), sin(theta_h) = Rb / r
+  float rho, r;              // the sample's rho and r
   float d;                   // distance from the texel's point along its ray
-  float dens_r, dens_m;      // Rayleigh and Mie densities x trapezoid weight
-  float tx, ty, tz;          // transmittance texel -> sample
+  float inv_2er;             // 1 / (2 r sin(theta_h) alpha_s), sin(theta_h) = Rb / r
+  F3 tr;                     // transmittance texel -> sample x Rayleigh density x weight
   float inv_range;           // 1 / (d_max - d_min) of the transmittance mapping
-  float pad[2];
+  F3 tm;                     // as tr, Mie
+  float pad;
+  int t0, t1;                // element offsets of the even and the odd one of the two
+  float w0, w1;              //   transmittance LUT rows around rho, and their weights
 };
 
-__host__ __device__ inline MultipleFastDims SingleDims(const Shape& s) {
-  int rows = kMultipleFastThreads / s.sw();
+// Rows of a block of `columns` texel columns, and samples per line stage.
+__host__ __device__ inline MultipleFastDims SingleDims(const Shape& s, int columns) {
+  int rows = columns / s.sw();
   rows = rows < 1 ? 1 : (rows > 4 ? 4 : rows);
-  if (s.tune[2] > 0) rows = s.tune[2];
+  if (s.tune[2] > 0 && (s.tune[2] < rows || columns > kSingleThreads)) rows = s.tune[2];
   int group = 32768 / (2 * 16 * rows * s.tw);
   group = group < 1 ? 1 : (group > 4 ? 4 : group);
   if (s.tune[3] > 0) group = s.tune[3];
   return MultipleFastDims{rows, group};
 }
 int SingleFastSmem(const Shape& s) {
-  const MultipleFastDims d = SingleDims(s);
+  const MultipleFastDims d = SingleDims(s, kSingleThreads);
+  return d.rows * kSingleSamples * (int)sizeof(SunSample) +
+         2 * d.group * d.rows * (s.tw + 1) * (int)sizeof(F3);
+}
+// The limit of the shapes and tunings taken: blocks of 256 columns, entries of
+// 16 bytes (no block needs more).
+int SingleFastLimit(const Shape& s) {
+  const MultipleFastDims d = SingleDims(s, kMultipleFastThreads);
   return d.rows * kSingleSamples * (int)sizeof(SunSample) + 2 * d.group * d.rows * s.tw * 16;
 }
 bool SingleFastFits(const Shape& s) {
-  return s.sw() <= kMultipleFastThreads * kMultipleFastMaxCols && SingleFastSmem(s) <= 48 * 1024;
+  return s.sw() <= kMultipleFastThreads * kMultipleFastMaxCols &&
+         SingleFastLimit(s) <= 48 * 1024;
 }
 int SingleFastTiles(const Shape& s) {
-  const int rows = SingleDims(s).rows;
+  const int rows = SingleDims(s, kSingleThreads).rows;
   return (s.sr * s.smu + rows - 1) / rows;
 }
 
@@ -1813,7 +1846,7 @@ bool FastTuningValid(const Shape& s, bool single, int rows, int group) {
   Shape t = s;
   t.tune[single ? 2 : 0] = rows;
   t.tune[single ? 3 : 1] = group;
-  return (single ? SingleFastSmem(t) : MultipleFastSmem(t)) <= 48 * 1024;
+  return (single ? SingleFastLimit(t) : MultipleFastSmem(t)) <= 48 * 1024;
 }
 
 // Sample i of the ray of LUT row `rowi` (the per-sample part of
@@ -1835,45 +1868,56 @@ __device__ SunSample MakeSunSample(const Instance& in, int rowi, int i) {
   const float fy = floorf(Y);
   const int j0 = ClampIdx((int)fy, s.th), j1 = ClampIdx((int)fy + 1, s.th);
   SunSample ss;
-  ss.t0 = j0 * s.tw;
-  ss.t1 = j1 * s.tw;
-  ss.b = Y - fy;
+  const float b = Y - fy;
+  const bool odd = j0 & 1;   // j1 is even (or j0 again, of weight b = 0)
+  ss.t0 = (odd ? j1 : j0) * s.tw;
+  ss.t1 = (odd ? j0 : j1) * s.tw;
+  ss.w0 = odd ? b : 1.0f - b;
+  ss.w1 = odd ? 1.0f - b : b;
   ss.rho = p.rho;
   ss.r = p.r;
-  ss.inv_r = 1.0f / p.r;
   // 1 / 0 = +inf for a point sun: the smoothstep then becomes a step at 0.
-  ss.inv_2e = 1.0f / (2.0f * (c.Rb / p.r * c.alpha_s));
+  ss.inv_2er = 1.0f / p.r * (1.0f / (2.0f * (c.Rb / p.r * c.alpha_s)));
   ss.d = d;
-  ss.dens_r = ProfileDensity(c.prof_r, p.h) * w;
-  ss.dens_m = ProfileDensity(c.prof_m, p.h) * w;
-  ss.tx = t.x;
-  ss.ty = t.y;
-  ss.tz = t.z;
+  ss.tr = t * (ProfileDensity(c.prof_r, p.h) * w);
+  ss.tm = t * (ProfileDensity(c.prof_m, p.h) * w);
   const float d_min = (c.H - p.rho) * (c.H + p.rho) / (c.Rt + p.r);
   ss.inv_range = 1.0f / (p.rho + c.H - d_min);
-  ss.pad[0] = ss.pad[1] = 0.0f;
+  ss.pad = 0.0f;
   return ss;
 }
 
-template <int kCols>
-__device__ __forceinline__ void SingleFastBlock(const Instance& in, int local, float4* smem) {
+// Up to kCols texel columns per thread; kBuild: the line columns a thread keeps
+// in registers.  kThreads: of the block, 0 where the launch says how many (any
+// number gives the same LUTs).
+template <int kCols, int kBuild, int kThreads>
+__device__ __forceinline__ void SingleFastBlock(const Instance& in, int local, float4* smem,
+                                                float magic) {
   const Shape s = in.s;
   const Consts& c = in.c;
-  const MultipleFastDims dims = SingleDims(s);
+  const MultipleFastDims dims = SingleDims(s, kSingleThreads);
+  const int threads = kThreads > 0 ? kThreads : (int)blockDim.x;
   const int W = s.sw(), R = dims.rows, G = dims.group, TW = s.tw;
   const int rows_total = s.sr * s.smu;
   [[maybe_unused]] const long long nT = s.t_texels();   // checked build
   const int row0 = local * R;
   SunSample* samp = reinterpret_cast<SunSample*>(smem);                       // [R][51]
-  float4* line = smem + R * kSingleSamples * (int)(sizeof(SunSample) / 16);   // [2][G][R][TW]
+  // [2][G][R][TW + 1] entries of three floats; entry 0 of a line is below its
+  // first column, for the tap of weight 0 there.
+  float* line = reinterpret_cast<float*>(smem + R * kSingleSamples * (int)(sizeof(SunSample) / 16));
+  const int line_floats = 3 * (TW + 1);
 
-  for (int e = threadIdx.x; e < R * kSingleSamples; e += kMultipleFastThreads) {
+  for (int e = threadIdx.x; e < 2 * G * R * 3; e += threads)
+    line[e / 3 * line_floats + e % 3] = 0.0f;
+  for (int e = threadIdx.x; e < R * kSingleSamples; e += threads) {
     const int rr = e / kSingleSamples, i = e - rr * kSingleSamples;
     if (row0 + rr < rows_total) samp[e] = MakeSunSample(in, row0 + rr, i);
   }
 
-  const int rr = kCols == 1 ? (int)threadIdx.x / W : 0;
-  const int x_t = kCols == 1 ? (int)threadIdx.x - rr * W : (int)threadIdx.x;
+  // Threads per row: a row's columns are x_t, x_t + stride, ...
+  const int stride = R == 1 ? threads : W;
+  const int rr = (int)threadIdx.x / stride;
+  const int x_t = (int)threadIdx.x - rr * stride;
   const int rowi = row0 + rr;
   const bool active = rr < R && rowi < rows_total;
   const int nmax = W - 1;
@@ -1883,8 +1927,8 @@ __device__ __forceinline__ void SingleFastBlock(const Instance& in, int local, f
     const TexelRow row = in.tab.rows[rowi];
 #pragma unroll
     for (int m = 0; m < kCols; ++m) {
-      const int x = min(x_t + m * kMultipleFastThreads, nmax);
-      const int n = x / s.smus, col = x - n * s.smus;
+      const int x = min(x_t + m * stride, nmax);
+      const int col = x / s.snu, n = x - col * s.snu;
       const TexelAngles ang = MakeAngles(s, row, in.tab.cols[col], n);
       rmu_s[m] = row.r * ang.mu_s;
       nu[m] = ang.nu;
@@ -1896,37 +1940,49 @@ __device__ __forceinline__ void SingleFastBlock(const Instance& in, int local, f
 
   const float H = c.H, H2 = c.H * c.H;
   const float tw1 = float(TW - 1);
-  const int line_stride = G * R * TW;
+  const uint32_t last = ((uint32_t)TW + (uint32_t)__float_as_int(magic)) * 12u;
+  const int line_stride = G * R * line_floats;
   const int stages = (kSingleSamples + G - 1) / G;
+  int o0 = -1, o1 = -1;
+  float4 ra[kBuild], rb[kBuild];
+#pragma unroll
+  for (int k = 0; k < kBuild; ++k) ra[k] = rb[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   for (int stage = 0; stage < stages; ++stage) {
-    float4* buf = line + (stage & 1) * line_stride;
+    float* buf = line + (stage & 1) * line_stride;
     const int first = stage * G;
     const int count = min(G, kSingleSamples - first);
-    // Transmittance LUT rows j0, j1 of each sample, interpolated in rho.
-    if (R == 1 && TW <= kMultipleFastThreads) {
-      // One row per block, one line column per thread: consecutive samples
-      // of the ray read the same two LUT rows 39% of the time at the
-      // reference's shape, and those rows, already in registers, are not
-      // loaded again (predicated loads: the same values, hence the same LUTs).
-      // Handling the samples that share one row as well (another 53%) with
-      // a branch per case, or with selects, measured slower.
-      const int x = threadIdx.x;
-      if (x < TW && row0 < rows_total) {
-        // The thread's columns addressed once, as in multiple scattering.
-        int o0 = -1, o1 = -1;
-        float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), b = a;
-        const float4* col = in.T + x;
-        float4* out_col = buf + x;
+    // The two transmittance LUT rows of each sample, interpolated in rho.
+    if (R == 1 && TW <= threads * kBuild) {
+      // One row per block, kBuild line columns per thread.  The thread keeps
+      // its columns of the last even and the last odd row in registers: of the
+      // rows around consecutive samples of a ray only 0.7 per sample are new
+      // at the reference's shape (predicated loads).
+      const int x = threadIdx.x, x_in = min(x, TW - 1);
+      if (row0 < rows_total) {
+        const float4* col = in.T + x_in;
+        float* out = buf + 3 * (x + 1);
         const SunSample* srow = samp + first;
         for (int g = 0; g < count; ++g) {
-          const SunSample& sm = srow[g];
-          const int fresh = (sm.t0 != o0) | (sm.t1 != o1);
-          LoadIf(a, ATMO_LINE_PTR(col, sm.t0, 0, nT - x), fresh);
-          LoadIf(b, ATMO_LINE_PTR(col, sm.t1, 0, nT - x), fresh);
-          o0 = sm.t0;
-          o1 = sm.t1;
-          out_col[g * TW] = make_float4(fmaf(sm.b, b.x - a.x, a.x), fmaf(sm.b, b.y - a.y, a.y),
-                                        fmaf(sm.b, b.z - a.z, a.z), 0.0f);
+          const int4 v = *reinterpret_cast<const int4*>(&srow[g].t0);
+          const float w0 = __int_as_float(v.z), w1 = __int_as_float(v.w);
+#pragma unroll
+          for (int k = 0; k < kBuild; ++k) {
+            const int xk = k * threads;
+            const bool mine = x + xk < TW;
+            LoadIf(ra[k], ATMO_LINE_PTR(col, v.x, mine ? xk : 0, nT - x_in), mine && v.x != o0);
+            LoadIf(rb[k], ATMO_LINE_PTR(col, v.y, mine ? xk : 0, nT - x_in), mine && v.y != o1);
+          }
+          o0 = v.x;
+          o1 = v.y;
+#pragma unroll
+          for (int k = 0; k < kBuild; ++k) {
+            if (x + k * threads < TW) {
+              out[3 * k * threads] = fmaf(w1, rb[k].x, w0 * ra[k].x);
+              out[3 * k * threads + 1] = fmaf(w1, rb[k].y, w0 * ra[k].y);
+              out[3 * k * threads + 2] = fmaf(w1, rb[k].z, w0 * ra[k].z);
+            }
+          }
+          out += line_floats;
         }
       }
     } else {
@@ -1934,12 +1990,14 @@ __device__ __forceinline__ void SingleFastBlock(const Instance& in, int local, f
         for (int q = 0; q < R; ++q) {
           if (row0 + q >= rows_total) break;
           const SunSample& sm = samp[q * kSingleSamples + first + g];
-          float4* out = buf + (g * R + q) * TW;
-          for (int x = threadIdx.x; x < TW; x += kMultipleFastThreads) {
+          float* line_q = buf + (g * R + q) * line_floats;
+          for (int x = threadIdx.x; x < TW; x += threads) {
             const float4 a = __ldg(ATMO_LINE_PTR(in.T, sm.t0, x, nT));
             const float4 b = __ldg(ATMO_LINE_PTR(in.T, sm.t1, x, nT));
-            out[x] = make_float4(fmaf(sm.b, b.x - a.x, a.x), fmaf(sm.b, b.y - a.y, a.y),
-                                 fmaf(sm.b, b.z - a.z, a.z), 0.0f);
+            float* out = line_q + 3 * (x + 1);
+            out[0] = fmaf(sm.w1, b.x, sm.w0 * a.x);
+            out[1] = fmaf(sm.w1, b.y, sm.w0 * a.y);
+            out[2] = fmaf(sm.w1, b.z, sm.w0 * a.z);
           }
         }
       }
@@ -1948,39 +2006,36 @@ __device__ __forceinline__ void SingleFastBlock(const Instance& in, int local, f
     if (active) {
       for (int g = 0; g < count; ++g) {
         const SunSample& sm = samp[rr * kSingleSamples + first + g];
-        const float4* L = buf + (g * R + rr) * TW;
+        // The line's last column, less the bits of the magic.
+        const uint32_t row =
+            (uint32_t)__cvta_generic_to_shared(buf + (g * R + rr) * line_floats) + last;
 #pragma unroll
         for (int m = 0; m < kCols; ++m) {
-          if (kCols > 1 && x_t + m * kMultipleFastThreads >= W) break;
+          if (x_t + m * stride >= W) break;
           // GetTransmittanceToSun (functions.glsl:552-563) at the sample, with
           // the lookup mapping of TransmittanceCoords.
           const float rmu = clampf(fmaf(sm.d, nu[m], rmu_s[m]), -sm.r, sm.r);
           // smoothstep(-e, e, mu_s - cos(theta_h)), cos(theta_h) = -rho / r.
-          const float st = clampf((rmu + sm.rho) * sm.inv_r * sm.inv_2e + 0.5f, 0.0f, 1.0f);
-          const float sun = st * st * fmaf(-2.0f, st, 3.0f);
-          const float delta = (sm.rho - rmu) * (sm.rho + rmu);
-          // H^2 - delta: zero, or a difference of floats far above FP32's
-          // normal range (normal); delta and rho - rmu: zero, or sums and
-          // products of lengths whose exact values are multiples of their
-          // operands' ulps (normal); H + sq >= H.
-          const float sq = SqrtFtz(fmaxf(H2 - delta, 0.0f));
-          const float rho_minus_a =
-              rmu < 0.0f ? (sm.rho - rmu > 0.0f ? DivFtz(delta, sm.rho - rmu) : 0.0f)
-                         : sm.rho + rmu;
-          const float omx =
-              clampf((rho_minus_a + DivFtz(delta, H + sq)) * sm.inv_range, 0.0f, 1.0f);
-          const float Xc = omx * tw1;
-          const float f = floorf(Xc);
-          const float gw = Xc - f;   // weight of the lower column
-          const int i_hi = TW - 1 - (int)f;
-          const int i_lo = max(i_hi - 1, 0);
-          const float4 lo = L[ATMO_CHECKED_INDEX(kCheckLineTap, i_lo, TW)];
-          const float4 hi = L[ATMO_CHECKED_INDEX(kCheckLineTap, max(i_hi, 0), TW)];
-          const F3 tsun{fmaf(gw, lo.x - hi.x, hi.x), fmaf(gw, lo.y - hi.y, hi.y),
-                        fmaf(gw, lo.z - hi.z, hi.z)};
-          const F3 t = F3{sm.tx, sm.ty, sm.tz} * (tsun * sun);
-          sum_r[m] = fma3(t, sm.dens_r, sum_r[m]);
-          sum_m[m] = fma3(t, sm.dens_m, sum_m[m]);
+          const float up = sm.rho + rmu, down = sm.rho - rmu;
+          const float st = FmaSat(up, sm.inv_2er, 0.5f);
+          // A sample in the planet's shadow adds nothing.
+          if (st > 0.0f) {
+            // With rho^2 - (r mu)^2 = up down, the distance to the top boundary
+            // less its least value is up + up down / (H + sq).  H^2 - up down:
+            // zero, or a difference of floats far above FP32's normal range
+            // (normal); up and down: zero, or sums of lengths whose exact values
+            // are multiples of their operands' ulps (normal); H + sq >= H.
+            const float sq = SqrtFtz(fmaxf(fmaf(-up, down, H2), 0.0f));
+            const float x = FmaSat(fmaf(up, DivFtz(down, H + sq), up), sm.inv_range, 0.0f);
+            const float cell = __fmaf_rd(x, tw1, magic);
+            const float gw = fmaf(x, tw1, magic - cell);   // weight of the lower column
+            const uint32_t at = row + (uint32_t)__float_as_int(cell) * (uint32_t)-12;
+            const F3 lo = LoadShared3<-12>(at), hi = LoadShared3<0>(at);
+            const F3 tsun = F3{fmaf(gw, lo.x - hi.x, hi.x), fmaf(gw, lo.y - hi.y, hi.y),
+                               fmaf(gw, lo.z - hi.z, hi.z)} * (st * st * fmaf(-2.0f, st, 3.0f));
+            sum_r[m] = fma3(tsun, sm.tr, sum_r[m]);
+            sum_m[m] = fma3(tsun, sm.tm, sum_m[m]);
+          }
         }
       }
     }
@@ -1990,30 +2045,47 @@ __device__ __forceinline__ void SingleFastBlock(const Instance& in, int local, f
   const float dx = in.tab.rows[rowi].d / float(kSingleScatteringSamples);
 #pragma unroll
   for (int m = 0; m < kCols; ++m) {
-    const int x = x_t + m * kMultipleFastThreads;
-    if (kCols > 1 && x >= W) break;
-    StoreSingleScattering(in, (long long)rowi * W + x, sum_r[m] * dx * c.solar * c.rayleigh,
+    const int x = x_t + m * stride;
+    if (x >= W) break;
+    const int col = x / s.snu, n = x - col * s.snu;
+    StoreSingleScattering(in, (long long)rowi * W + n * s.smus + col, sum_r[m] * dx * c.solar * c.rayleigh,
                           sum_m[m] * dx * c.solar * c.mie_sca);
   }
 }
 
-// 4 blocks per SM (64 registers, a few spills) beat 3 at 75 registers by 10%.
-__global__ void __launch_bounds__(kMultipleFastThreads, 4)
-k_single_fast(const Instance* __restrict__ insts, WorkList wl) {
+// A kernel per SingleKind, so that each has the registers it needs: one column
+// per thread up to 128 columns (64 registers), two up to 256 (72, 7 blocks of
+// 128 threads per SM; 6 blocks take 1% and 8 take 3% longer), four above (64, 4
+// blocks; 3 take 12% longer).
+template <int kKind>
+__global__ void __launch_bounds__(kKind == kSingleTwo ? kSingleThreads : kMultipleFastThreads,
+                                  kKind == kSingleTwo ? 7 : 4)
+k_single_fast(const Instance* __restrict__ insts, WorkList wl, float magic) {
   extern __shared__ float4 smem[];
   int local;
   const Instance& in = insts[FindEntry(wl, blockIdx.x, &local)];
-  if (in.s.sw() <= kMultipleFastThreads) {
-    SingleFastBlock<1>(in, local, smem);
-  } else {
-    SingleFastBlock<kMultipleFastMaxCols>(in, local, smem);
-  }
+  if (SingleKind(in.s) != kKind) return;
+  if (kKind == kSingleOne) SingleFastBlock<1, 2, 0>(in, local, smem, magic);
+  if (kKind == kSingleTwo) SingleFastBlock<2, 2, kSingleThreads>(in, local, smem, magic);
+  if (kKind == kSingleFour) SingleFastBlock<4, 2, kMultipleFastThreads>(in, local, smem, magic);
 }
 
 cudaError_t LaunchSingleFast(const Instance* insts, WorkList wl, int tiles, int smem_bytes,
                              cudaStream_t st) {
   // smem_bytes: the largest SingleFastSmem of the work list's instances.
-  k_single_fast<<<tiles, kMultipleFastThreads, (size_t)smem_bytes, st>>>(insts, wl);
+  const size_t bytes = (size_t)smem_bytes;
+  if (wl.kinds & kSingleOne) {
+    // Where every block of the launch is resident at once (4 per SM), threads
+    // without a texel column help with the samples and the lines: one instance
+    // of half size (1024 rows of 64 columns) 43 us against 51; 8 of them 260
+    // us against 234.
+    const int threads = tiles <= 4 * 152 ? kMultipleFastThreads : kSingleThreads;
+    k_single_fast<kSingleOne><<<tiles, threads, bytes, st>>>(insts, wl, kRoundMagic);
+  }
+  if (wl.kinds & kSingleTwo)
+    k_single_fast<kSingleTwo><<<tiles, kSingleThreads, bytes, st>>>(insts, wl, kRoundMagic);
+  if (wl.kinds & kSingleFour)
+    k_single_fast<kSingleFour><<<tiles, kMultipleFastThreads, bytes, st>>>(insts, wl, kRoundMagic);
   return cudaGetLastError();
 }
 

@@ -72,7 +72,18 @@ ATMO_HD int DensityKind(const Shape& s) {
   if (s.snu > 16 || s.iw > 512 || texels < (s.snu <= 5 ? 49152 : 131072)) return kDensityLookups;
   return s.snu <= 4 || texels < 262144 ? kDensityArcs4 : kDensityArcs8;
 }
-ATMO_HD int KernelKinds(const Shape& s) { return MultipleKind(s) | DensityKind(s); }
+// The single-scattering kernel of a LUT shape, a bit: one, two or four texel
+// columns of a row per thread.  Two share a sample's loads and hide each
+// other's latency; a row of up to 128 columns has one for every thread of a block (one
+// instance of 64 columns: 57 us with one per thread, 76 with two).
+constexpr int kSingleOne = 64, kSingleTwo = 128, kSingleFour = 256;
+ATMO_HD int SingleKind(const Shape& s) {
+  return s.sw() <= 128 ? kSingleOne : s.sw() <= 256 ? kSingleTwo : kSingleFour;
+}
+
+ATMO_HD int KernelKinds(const Shape& s) {
+  return MultipleKind(s) | DensityKind(s) | SingleKind(s);
+}
 
 #ifdef __CUDACC__
 // Finds the work-list entry holding `tile` (binary search over start[]).
