@@ -1118,13 +1118,16 @@ constexpr int kMultipleFastMaxCols = 4;   // texel columns per thread (W <= 1024
 constexpr int kRaySamples = kMultipleScatteringSamples + 1;
 
 struct __align__(16) RaySample {
-  int r00, r01, r10, r11;    // element offsets of the LUT rows (k0 j0, k0 j1, k1 j0, k1 j1)
+  // Element offsets of the four LUT rows around the sample, the (k, j) = (r,
+  // mu) row with even k and j first, then odd j, odd k, both odd: of two
+  // samples' rows, those they share have the same place.
+  int r00, r01, r10, r11;
   float w00, w01, w10, w11;  // their bilinear weights in (mu, r)
   float tx, ty, tz;          // transmittance texel -> sample x dx x trapezoid weight
+  float rb_inv_r, rb_d;      // Rb / r and Rb d / r at the sample
+  int fresh;                 // a bit for each row that the next sample changes
   float d;                   // distance from the texel's point along its ray
   float inv_r;               // 1 / r at the sample
-  float pad;
-  float rb_inv_r, rb_d;      // Rb / r and Rb d / r at the sample
 };
 
 struct MultipleFastDims {
@@ -1173,14 +1176,18 @@ __device__ RaySample MakeRaySample(const Instance& in, int rowi, int i) {
   const int k0 = ClampIdx((int)fz, s.sr), k1 = ClampIdx((int)fz + 1, s.sr);
   const int W = s.sw();
   RaySample rs;
-  rs.r00 = (k0 * s.smu + j0) * W;
-  rs.r01 = (k0 * s.smu + j1) * W;
-  rs.r10 = (k1 * s.smu + j0) * W;
-  rs.r11 = (k1 * s.smu + j1) * W;
-  rs.w00 = (1.0f - b) * (1.0f - cz);
-  rs.w01 = b * (1.0f - cz);
-  rs.w10 = (1.0f - b) * cz;
-  rs.w11 = b * cz;
+  const bool oj = j0 & 1, ok = k0 & 1;
+  const int je = oj ? j1 : j0, jo = oj ? j0 : j1, ke = ok ? k1 : k0, ko = ok ? k0 : k1;
+  const float bo = oj ? 1.0f - b : b, be = oj ? b : 1.0f - b;
+  const float co = ok ? 1.0f - cz : cz, ce = ok ? cz : 1.0f - cz;
+  rs.r00 = (ke * s.smu + je) * W;
+  rs.r01 = (ke * s.smu + jo) * W;
+  rs.r10 = (ko * s.smu + je) * W;
+  rs.r11 = (ko * s.smu + jo) * W;
+  rs.w00 = be * ce;
+  rs.w01 = bo * ce;
+  rs.w10 = be * co;
+  rs.w11 = bo * co;
   const float dw = dx * w;
   rs.tx = t.x * dw;
   rs.ty = t.y * dw;
@@ -1189,7 +1196,7 @@ __device__ RaySample MakeRaySample(const Instance& in, int rowi, int i) {
   rs.inv_r = 1.0f / p.r;
   rs.rb_inv_r = c.Rb / p.r;
   rs.rb_d = rs.rb_inv_r * d;
-  rs.pad = 0.0f;
+  rs.fresh = 0;
   return rs;
 }
 
@@ -1390,20 +1397,25 @@ __device__ __forceinline__ void MultipleFastBlock(const Instance& in, int local,
 // A texel whose nu is not clamped sits on its own node, so its taps are in
 // its own warp.  The texels of a row and column whose nu is clamped share the
 // clamped value (one below, one above the physical range), which lies between
-// two nodes n0, n0 + 1: the lanes of column c in those two nodes' warps each
-// march that nu through their own node's line, weighted with the node's lerp
-// weight, and the two parts are added through shared memory at the end.  A
-// lane's work is thus up to three of {its own texel, the low and the high
-// clamped nu}, put in up to three slots; a slot is marched when any lane of
-// the warp uses it (1.7 of them on average at the reference's shape).
+// two nodes n0, n0 + 1: those two nodes' warps each march that nu through
+// their own node's line, weighted with the node's lerp weight, and the two
+// parts are added through shared memory at the end.  A column thus gives its
+// warp up to three of the tasks {its own texel, the low and the high clamped
+// nu}, 1.2 on average at the reference's shape.  Any lane can march any task,
+// so the warp packs them: 1.5 marches of 32 tasks per node, where a lane that
+// marches its own columns' tasks needs 1.7.
 //
-// Bound by instruction issue (70%) and the L1 data pipe (75%) together: 111
-// instructions and 31 wavefronts per warp and sample, against 135 and 45 of
+// Bound by the L1 data pipe (78%) and instruction issue (74%) together, 27
+// wavefronts and 97 instructions per warp and sample, against 45 and 135 of
 // the lines in shared memory, whose stores, taps and clamps it does without.
-// Per 16-instance launch at the reference's shape 4.13 -> 3.26 ms; one
-// high-resolution instance 4.40 -> 3.37 ms.
+// Of a sample's four rows those it shares with the last one stay in
+// registers.  Per 16-instance launch at the reference's shape 4.13 (lines in
+// shared memory) -> 3.25 (nodes) -> 3.08 (packed tasks) -> 2.95 (four items
+// per warp, handed out) -> 2.76 ms (shared rows kept); one high-resolution
+// instance 4.40 -> 3.43 -> 3.08 -> 3.03 -> 2.73 ms.
 // ---------------------------------------------------------------------------
 constexpr int kNodeWarps = kMultipleFastThreads / 32;
+constexpr int kNodeSamples = kRaySamples + 1;   // the last one twice
 __host__ __device__ inline bool MultipleByNodes(const Shape& s) { return MultipleKind(s) < 4; }
 // Nu nodes held by one warp, and warp items (of that many nodes) per row.
 __host__ __device__ inline int NodesPerWarp(const Shape& s) {
@@ -1413,17 +1425,16 @@ __host__ __device__ inline int NodeItemsPerRow(const Shape& s) {
   const int per = NodesPerWarp(s);
   return (s.snu + per - 1) / per;
 }
-// Rows per block: as many (up to 4) as give its 8 warps one item each, or two
-// where that leaves two full waves of blocks (4 per SM on 152 SMs).  Two items
-// per warp halve the blocks' idle time (their sample tables are built by 51
-// threads per row, and the warps of the outermost nodes have less to do):
-// 3.26 ms per 16-instance launch at the reference's shape against 3.37 with
-// one (four give 3.22 but too few blocks for a single instance); smaller LUTs
-// want the shorter blocks.
+// Rows per block: as many (up to 4) as give its 8 warps one item each, or four
+// where that leaves a full wave of blocks (4 per SM on 152 SMs).  Four items
+// per warp shorten the blocks' idle time (their sample tables are built by 51
+// threads per row, and the items differ): 2.82 ms per 16-instance launch at
+// the reference's shape against 2.91 with two; smaller LUTs want the shorter
+// blocks.
 __host__ __device__ inline int NodeRows(const Shape& s) {
   const int items = NodeItemsPerRow(s);
-  const bool many = (long long)s.sr * s.smu * items >= 2LL * 2 * kNodeWarps * 4 * 152;
-  const int rows = (many ? 2 : 1) * kNodeWarps / items;
+  const bool many = (long long)s.sr * s.smu * items >= 4LL * kNodeWarps * 4 * 152;
+  const int rows = (many ? 4 : 1) * kNodeWarps / items;
   return rows < 1 ? 1 : (rows > 4 ? 4 : rows);
 }
 
@@ -1458,11 +1469,12 @@ __device__ __forceinline__ float SunCoordinate(const SunMap& m, float rmus) {
   return FmaSat(q, m.k1, m.k0);
 }
 
-// A 256-bit read-only load of two neighbouring texels (32-byte aligned).
-__device__ __forceinline__ void LoadTwo(float4& a, float4& b, const float4* ptr) {
-  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-      : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
-      : "l"(ptr));
+// LoadIf of two neighbouring texels (32-byte aligned).
+__device__ __forceinline__ void LoadTwoIf(float4& a, float4& b, const float4* ptr, int p) {
+  asm("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %9, 0;\n\t"
+      "@q ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n\t}"
+      : "+f"(a.x), "+f"(a.y), "+f"(a.z), "+f"(a.w), "+f"(b.x), "+f"(b.y), "+f"(b.z), "+f"(b.w)
+      : "l"(ptr), "r"(p));
 }
 
 // A lane's columns of one LUT row: one, two with a 256-bit load (kPair: the
@@ -1473,15 +1485,15 @@ struct NodeRow {
   float4 v[kCols];
 };
 template <int kCols, bool kPair>
-__device__ __forceinline__ void LoadRow(NodeRow<kCols>& row, const float4* col, int offset,
-                                        int second, [[maybe_unused]] long long n) {
+__device__ __forceinline__ void LoadRowIf(NodeRow<kCols>& row, const float4* col, int offset,
+                                          int second, [[maybe_unused]] long long n, int p) {
   if constexpr (kCols == 1) {
-    row.v[0] = __ldg(ATMO_LINE_PTR(col, offset, 0, n));
+    LoadIf(row.v[0], ATMO_LINE_PTR(col, offset, 0, n), p);
   } else if constexpr (kPair) {
-    LoadTwo(row.v[0], row.v[1], ATMO_LINE_PTR(col, offset, 0, n - 1));
+    LoadTwoIf(row.v[0], row.v[1], ATMO_LINE_PTR(col, offset, 0, n - 1), p);
   } else {
-    row.v[0] = __ldg(ATMO_LINE_PTR(col, offset, 0, n));
-    row.v[1] = __ldg(ATMO_LINE_PTR(col, offset, second, n));
+    LoadIf(row.v[0], ATMO_LINE_PTR(col, offset, 0, n), p);
+    LoadIf(row.v[1], ATMO_LINE_PTR(col, offset, second, n), p);
   }
 }
 
@@ -1490,73 +1502,75 @@ __device__ __forceinline__ F3 Shuffle3(F3 v, int lane) {
             __shfl_sync(0xffffffffu, v.z, lane)};
 }
 
-// The line at x of the mu_s range of the lane's node.  magic: kRoundMagic
-// plus the node's first lane; the FMA rounded down leaves the lower tap's
-// lane in the sum's low bits (a shuffle's lane counts modulo 32: at x = 1 the
-// upper tap, of weight 0, may be any lane).
+// acc + the line at x of the mu_s range of a node.  magic: kRoundMagic plus
+// the node's first lane; the FMA rounded down leaves the lower tap's lane in
+// the sum's low bits (a shuffle's lane counts modulo 32: at x = 1 the upper
+// tap, of weight 0, may be any lane).
 template <int kCols>
-__device__ __forceinline__ F3 TapLine(const F3 (&line)[kCols], float x, float n1, float magic) {
+__device__ __forceinline__ F3 TapLine(const F3 (&line)[kCols], float x, float n1, float magic,
+                                      F3 acc) {
   const float t = __fmaf_rd(x, n1, magic);
   const float w1 = fmaf(x, n1, magic - t), w0 = 1.0f - w1;
   const int i0 = __float_as_int(t);
   if constexpr (kCols == 1) {
     const F3 t0 = Shuffle3(line[0], i0), t1 = Shuffle3(line[0], i0 + 1);
-    return fma3(t1, w1, t0 * w0);
+    return fma3(t1, w1, fma3(t0, w0, acc));
   } else {
     // Columns 2 l, 2 l + 1 in lane l: the taps i0, i0 + 1 are one even and
     // one odd column.
     const bool odd = i0 & 1;
     const F3 te = Shuffle3(line[0], (i0 + 1) >> 1), to = Shuffle3(line[1], i0 >> 1);
-    return fma3(to, odd ? w0 : w1, te * (odd ? w1 : w0));
+    return fma3(to, odd ? w0 : w1, fma3(te, odd ? w1 : w0, acc));
   }
 }
 
-// Marches the row's samples: acc[s][m] += the line's value at the nu of slot
-// s of the lane's column m, times the sample's transmittance and weight.
-template <int kCols, int kSlots, bool kPair>
+// Marches the row's samples: acc[t] += the line's value at the mu_s and nu of
+// the lane's task t, times the sample's transmittance and weight.
+template <int kCols, int kTasks, bool kPair, bool kSub>
 __device__ __forceinline__ void MarchNodes(const RaySample* samp, const float4* col, int second,
-                                           long long n, const SunMap& map, float magic,
-                                           const float (&rmu_s)[kCols],
-                                           const float (&nu)[kSlots][kCols],
-                                           F3 (&acc)[kSlots][kCols]) {
+                                           long long n, const SunMap& map,
+                                           const float (&magic)[kSub ? kTasks : 1],
+                                           const float (&rmu_s)[kTasks],
+                                           const float (&nu)[kTasks], F3 (&acc)[kTasks]) {
   NodeRow<kCols> a, b, p, q;
-  int4 r = *reinterpret_cast<const int4*>(&samp[0].r00);
-  LoadRow<kCols, kPair>(a, col, r.x, second, n);
-  LoadRow<kCols, kPair>(b, col, r.y, second, n);
-  LoadRow<kCols, kPair>(p, col, r.z, second, n);
-  LoadRow<kCols, kPair>(q, col, r.w, second, n);
+#pragma unroll
+  for (int m = 0; m < kCols; ++m)
+    a.v[m] = b.v[m] = p.v[m] = q.v[m] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  const int4 r = *reinterpret_cast<const int4*>(&samp[0].r00);
+  LoadRowIf<kCols, kPair>(a, col, r.x, second, n, 1);
+  LoadRowIf<kCols, kPair>(b, col, r.y, second, n, 1);
+  LoadRowIf<kCols, kPair>(p, col, r.z, second, n, 1);
+  LoadRowIf<kCols, kPair>(q, col, r.w, second, n, 1);
 #pragma unroll 1
   for (int i = 0; i < kRaySamples; ++i) {
     const float4 w = *reinterpret_cast<const float4*>(&samp[i].w00);
+    const float4 t = *reinterpret_cast<const float4*>(&samp[i].tx);
+    const float2 rb_fresh = *reinterpret_cast<const float2*>(&samp[i].rb_d);
+    const int fresh = __float_as_int(rb_fresh.y);
     F3 line[kCols];
 #pragma unroll
     for (int m = 0; m < kCols; ++m) {
       line[m] = fma3(f3(q.v[m]), w.w,
-                     fma3(f3(p.v[m]), w.z, fma3(f3(b.v[m]), w.y, f3(a.v[m]) * w.x)));
+                     fma3(f3(p.v[m]), w.z, fma3(f3(b.v[m]), w.y, f3(a.v[m]) * w.x))) *
+                F3{t.x, t.y, t.z};
     }
-    // The next sample's rows are loaded while this one's taps are made; a
-    // sample in the same cell (r00 and r11 fix all four rows) keeps them.
-    if (i + 1 < kRaySamples) {
+    // The next sample's rows are loaded while this one's taps are made, but
+    // for those it shares with this one (sample 51 is sample 50 again).  One
+    // column per lane skips them all with a branch where there is nothing to
+    // load (2.76 ms per 16-instance launch against 2.82; two columns per lane
+    // 2.80 against 2.79).
+    if (kCols == 2 || fresh) {
       const int4 r1 = *reinterpret_cast<const int4*>(&samp[i + 1].r00);
-      if (r1.x != r.x || r1.w != r.w) {
-        LoadRow<kCols, kPair>(a, col, r1.x, second, n);
-        LoadRow<kCols, kPair>(b, col, r1.y, second, n);
-        LoadRow<kCols, kPair>(p, col, r1.z, second, n);
-        LoadRow<kCols, kPair>(q, col, r1.w, second, n);
-        r = r1;
-      }
+      LoadRowIf<kCols, kPair>(a, col, r1.x, second, n, fresh & 1);
+      LoadRowIf<kCols, kPair>(b, col, r1.y, second, n, fresh & 2);
+      LoadRowIf<kCols, kPair>(p, col, r1.z, second, n, fresh & 4);
+      LoadRowIf<kCols, kPair>(q, col, r1.w, second, n, fresh & 8);
     }
     // Rb mu_s at the sample: (r mu_s + d nu) Rb / r_i.
-    const float3 t{samp[i].tx, samp[i].ty, samp[i].tz};
-    const float2 rb = *reinterpret_cast<const float2*>(&samp[i].rb_inv_r);
 #pragma unroll
-    for (int m = 0; m < kCols; ++m) {
-      const float rmus = rmu_s[m] * rb.x;
-#pragma unroll
-      for (int s = 0; s < kSlots; ++s) {
-        const float x = SunCoordinate(map, fmaf(nu[s][m], rb.y, rmus));
-        acc[s][m] = fma3(TapLine<kCols>(line, x, map.n1, magic), F3{t.x, t.y, t.z}, acc[s][m]);
-      }
+    for (int k = 0; k < kTasks; ++k) {
+      const float x = SunCoordinate(map, fmaf(nu[k], rb_fresh.x, rmu_s[k] * t.w));
+      acc[k] = TapLine<kCols>(line, x, map.n1, magic[kSub ? k : 0], acc[k]);
     }
   }
 }
@@ -1583,119 +1597,135 @@ __device__ __forceinline__ void StoreMultiple(const Instance& in, int texel, F3 
   in.S[texel] = make_float4(o.x + add.x, o.y + add.y, o.z + add.z, o.w);
 }
 
-template <int kCols, bool kPair>
+// A task of a warp: the nu to march, and where its result goes: the lane and
+// column (lane x kCols + m) x 256 + 1 for the texel itself, 2 + 2 side + half
+// for a part of a clamped nu.
+struct NodeTask {
+  float nu;
+  int code;
+};
+
+template <int kCols, bool kPair, bool kSub>
 __device__ __forceinline__ void MultipleNodesBlock(const Instance& in, int local, float4* smem) {
   const Shape s = in.s;
   const Consts& c = in.c;
   const int W = s.sw(), R = NodeRows(s), per = NodesPerWarp(s), items = NodeItemsPerRow(s);
   const int rows_total = s.sr * s.smu, row0 = local * R;
   [[maybe_unused]] const long long nS = s.s_texels();   // checked build
-  RaySample* samp = reinterpret_cast<RaySample*>(smem);                        // [R][51]
-  float4* edge = smem + R * kRaySamples * (int)(sizeof(RaySample) / 16);       // [R][2][2][MU_S]
+  RaySample* samp = reinterpret_cast<RaySample*>(smem);                        // [R][52]
+  float4* edge = smem + R * kNodeSamples * (int)(sizeof(RaySample) / 16);       // [R][2][2][MU_S]
   const int lane = threadIdx.x & 31, warp = threadIdx.x / 32;
+  NodeTask* tasks = reinterpret_cast<NodeTask*>(edge + R * 4 * s.smus) +      // [8][3][32 kCols]
+                    warp * 96 * kCols;
+  __shared__ int next;   // the first item no warp has taken
+  if (threadIdx.x == 0) next = kNodeWarps;
 
-  for (int e = threadIdx.x; e < R * kRaySamples; e += kMultipleFastThreads) {
-    const int rr = e / kRaySamples, i = e - rr * kRaySamples;
+  for (int e = threadIdx.x; e < R * kNodeSamples; e += kMultipleFastThreads) {
+    const int rr = e / kNodeSamples, i = min(e - rr * kNodeSamples, kRaySamples - 1);
     if (row0 + rr < rows_total) samp[e] = MakeRaySample(in, RowAt(in.tab, row0 + rr), i);
   }
   for (int e = threadIdx.x; e < R * 4 * s.smus; e += kMultipleFastThreads)
     edge[e] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   __syncthreads();
+  for (int e = threadIdx.x; e < R * kNodeSamples - 1; e += kMultipleFastThreads) {
+    const int4 u = *reinterpret_cast<const int4*>(&samp[e].r00);
+    const int4 v = *reinterpret_cast<const int4*>(&samp[e + 1].r00);
+    samp[e].fresh = (u.x != v.x) | (u.y != v.y) << 1 | (u.z != v.z) << 2 | (u.w != v.w) << 3;
+  }
+  __syncthreads();
 
   const SunMap map = MakeSunMap(c, s);
   const float nodes1 = float(s.snu - 1);
-  for (int item = warp; item < R * items; item += kNodeWarps) {
-    const int rr = item / items;
-    if (row0 + rr >= rows_total) break;
-    // Rotated from row to row: the outermost nodes have the least work.
-    const int slot = (item + 3 * rr) % items;
+  // The items go to the warps as these finish, the innermost nodes (the most
+  // work) first.
+  for (int item = warp; item < R * items;) {
+    const int rr = item % R, o = item / R;
+    const int slot = (items - 1) / 2 + (o & 1 ? (o + 1) / 2 : -(o / 2));
+    if (lane == 0) item = atomicAdd(&next, 1);
+    item = __shfl_sync(0xffffffffu, item, 0);
+    if (row0 + rr >= rows_total) continue;
     const int rowi = RowAt(in.tab, row0 + rr);
-    const int sub = kCols == 1 ? lane / s.smus : 0;
+    const int sub = kSub ? lane / s.smus : 0;
     const int n = slot * per + sub;
     const int col0 = kCols == 1 ? lane - sub * s.smus : 2 * lane;
     const int cols = sub < per && n < s.snu ? min(max(s.smus - col0, 0), kCols) : 0;
     // Lanes without a texel march column 0 of node 0 and keep nothing.
     const int second = cols == 2 ? 1 : 0;
     const float4* col = in.dJ + (cols > 0 ? n * s.smus + col0 : 0);
-    float rmu_s[kCols], nu[3][kCols], weight[3][kCols];
-    int use[3][kCols], slots = 0;   // 0: none, 1: own texel, 2 + 2 side + half: clamped part
+    // The tasks of the warp's columns, packed: any lane can march any of them,
+    // as the taps are shuffles.
+    int count = 0;
+    auto add = [&](bool any, int m, int use, float nu) {
+      const unsigned mask = __ballot_sync(0xffffffffu, any);
+      if (any)
+        tasks[count + __popc(mask & ((1u << lane) - 1u))] =
+            NodeTask{nu, (lane * kCols + m) << 8 | use};
+      count += __popc(mask);
+    };
 #pragma unroll
     for (int m = 0; m < kCols; ++m) {
       const int colm = m < cols ? col0 + m : 0;
       const NodeNu own = TexelNu(in, rowi, colm, min(n, s.snu - 1));
-      rmu_s[m] = in.tab.rows[rowi].r * in.tab.cols[colm].mu_s;
-      int used = 0;
-#pragma unroll
-      for (int q = 0; q < 3; ++q) {
-        nu[q][m] = own.nu;
-        weight[q][m] = 1.0f;
-        use[q][m] = 0;
-      }
-      if (m < cols && own.side < 0) {
-        use[0][m] = 1;
-        used = 1;
-      }
+      add(m < cols && own.side < 0, m, 1, own.nu);
 #pragma unroll
       for (int side = 0; side < 2; ++side) {
-        const NodeNu end = TexelNu(in, rowi, colm, side == 0 ? 0 : s.snu - 1);
-        const float x = (end.nu + 1.0f) * 0.5f * nodes1, fx = floorf(x);
-        const int half = n - (int)fx;   // 0: the lower of the two nodes, 1: the upper
-        const float l1 = x - fx;
         // Some texel's nu is clamped at an end where the end node's own is.
-        if (m < cols && end.side == side && (half == 0 || half == 1)) {
-          const float w = half == 0 ? 1.0f - l1 : l1;
-#pragma unroll
-          for (int q = 0; q < 3; ++q) {
-            if (q == used) {
-              nu[q][m] = end.nu;
-              weight[q][m] = w;
-              use[q][m] = 2 + 2 * side + half;
-            }
-          }
-          ++used;
-        }
+        const NodeNu end = TexelNu(in, rowi, colm, side == 0 ? 0 : s.snu - 1);
+        const int half = n - (int)floorf((end.nu + 1.0f) * 0.5f * nodes1);
+        add(m < cols && end.side == side && (half == 0 || half == 1), m, 2 + 2 * side + half,
+            end.nu);
       }
-      slots = max(slots, used);
     }
-    slots = __reduce_max_sync(0xffffffffu, slots);
-    const RaySample* srow = samp + rr * kRaySamples;
-    const float magic = kRoundMagic + (kCols == 1 ? float(sub * s.smus) : 0.0f);
-    auto keep = [&](int m, int used, float w, float nu_m, F3 sum) {
-      if (used == 1) StoreMultiple(in, rowi * W + n * s.smus + col0 + m, sum, nu_m);
-      if (used >= 2) {
-        edge[(rr * 4 + used - 2) * s.smus + col0 + m] = to4(sum * w, 0.0f);
+    __syncwarp();
+    const RaySample* srow = samp + rr * kNodeSamples;
+    auto march = [&](auto per_lane, int first) {
+      constexpr int kTasks = decltype(per_lane)::value;
+      float magic[kSub ? kTasks : 1], rmu_s[kTasks], nu[kTasks];
+      F3 acc[kTasks];
+#pragma unroll
+      for (int k = 0; k < kTasks; ++k) {
+        const int t = first + 32 * k + lane;
+        const NodeTask task = t < count ? tasks[t] : NodeTask{0.0f, 0};
+        const int at = task.code >> 8, of = kSub ? at / s.smus * s.smus : 0;
+        nu[k] = task.nu;
+        rmu_s[k] = in.tab.rows[rowi].r * in.tab.cols[at - of].mu_s;
+        magic[kSub ? k : 0] = kRoundMagic + float(of);
+        acc[k] = f3(0.0f);
+      }
+      MarchNodes<kCols, kTasks, kPair, kSub>(srow, col, second, nS, map, magic, rmu_s, nu, acc);
+#pragma unroll
+      for (int k = 0; k < kTasks; ++k) {
+        const int t = first + 32 * k + lane;
+        if (t >= count) continue;
+        const NodeTask task = tasks[t];
+        const int at = task.code >> 8, use = task.code & 255;
+        if (use == 1) {
+          StoreMultiple(in, rowi * W + slot * per * s.smus + at, acc[k], task.nu);
+        } else {
+          const float x = (task.nu + 1.0f) * 0.5f * nodes1, l1 = x - floorf(x);
+          const int of = kSub ? at / s.smus * s.smus : 0;
+          edge[(rr * 4 + use - 2) * s.smus + at - of] =
+              to4(acc[k] * (use & 1 ? l1 : 1.0f - l1), 0.0f);
+        }
       }
     };
-    for (int first = 0; first < slots; first += 2) {
-      float nu2[2][kCols];
-      F3 acc[2][kCols];
-#pragma unroll
-      for (int m = 0; m < kCols; ++m) {
-        nu2[0][m] = first == 0 ? nu[0][m] : nu[2][m];
-        nu2[1][m] = nu[1][m];
-        acc[0][m] = acc[1][m] = f3(0.0f);
-      }
-      if (slots - first >= 2) {
-        MarchNodes<kCols, 2, kPair>(srow, col, second, nS, map, magic, rmu_s, nu2, acc);
+    for (int first = 0; first < count;) {
+      const int left = count - first;
+      if (kCols == 2 && left > 96) {
+        march(std::integral_constant<int, 4>(), first);
+        first += 128;
+      } else if (kCols == 2 && left > 64) {
+        march(std::integral_constant<int, 3>(), first);
+        first += 96;
+      } else if (left > 32) {
+        march(std::integral_constant<int, 2>(), first);
+        first += 64;
       } else {
-        float nu1[1][kCols];
-        F3 acc1[1][kCols];
-#pragma unroll
-        for (int m = 0; m < kCols; ++m) {
-          nu1[0][m] = nu2[0][m];
-          acc1[0][m] = f3(0.0f);
-        }
-        MarchNodes<kCols, 1, kPair>(srow, col, second, nS, map, magic, rmu_s, nu1, acc1);
-#pragma unroll
-        for (int m = 0; m < kCols; ++m) acc[0][m] = acc1[0][m];
-      }
-#pragma unroll
-      for (int m = 0; m < kCols; ++m) {
-        keep(m, first == 0 ? use[0][m] : use[2][m], first == 0 ? weight[0][m] : weight[2][m],
-             nu2[0][m], acc[0][m]);
-        if (first == 0) keep(m, use[1][m], weight[1][m], nu2[1][m], acc[1][m]);
+        march(std::integral_constant<int, 1>(), first);
+        first += 32;
       }
     }
+    __syncwarp();
   }
   __syncthreads();
 
@@ -1725,9 +1755,11 @@ k_multiple_nodes(const Instance* __restrict__ insts, WorkList wl) {
   const Instance& in = insts[FindEntry(wl, blockIdx.x, &local)];
   if (MultipleKind(in.s) != kCols) return;
   if (kCols == 2 && in.s.smus % 2 == 0 && ((size_t)in.dJ & 31) == 0) {
-    MultipleNodesBlock<kCols, kCols == 2>(in, local, smem);
+    MultipleNodesBlock<kCols, kCols == 2, false>(in, local, smem);
+  } else if (kCols == 1 && in.s.smus <= 16) {
+    MultipleNodesBlock<kCols, false, kCols == 1>(in, local, smem);
   } else {
-    MultipleNodesBlock<kCols, false>(in, local, smem);
+    MultipleNodesBlock<kCols, false, false>(in, local, smem);
   }
 }
 
@@ -1753,7 +1785,8 @@ int MultipleFastTiles(const Shape& s) {
 }
 int MultipleFastSmem(const Shape& s) {
   if (MultipleByNodes(s))
-    return NodeRows(s) * (kRaySamples * (int)sizeof(RaySample) + 4 * s.smus * 16);
+    return NodeRows(s) * (kNodeSamples * (int)sizeof(RaySample) + 4 * s.smus * 16) +
+           kNodeWarps * 96 * MultipleKind(s) * (int)sizeof(NodeTask);
   const MultipleFastDims d = MultipleDims(s);
   return d.rows * kRaySamples * (int)sizeof(RaySample) + 2 * d.group * d.rows * s.sw() * 16;
 }

@@ -47,16 +47,20 @@ struct WorkList {
 };
 
 // The multiple-scattering kernel of a LUT shape, a bit: 1, the mu_s columns of
-// a nu node in one register per lane (MU_S <= 32, where the 32 / MU_S nodes of
-// a warp fill 3/4 of its lanes); 2, in two (MU_S 33 to 64 and more than 256
-// columns in all); 4, lines in shared memory.  4 instances of 32 x 128 rows,
-// kernel 4 against the other, ms: MU_S x NU = 8 x 8 0.301 / 0.244, 32 x 8
-// 1.10 / 0.87, 11 x 8 (22 lanes) 0.439 / 0.461, 19 x 8 (19 lanes) 0.766 /
-// 0.844; 40 x 8 1.99 / 1.66, 64 x 8 2.40 / 1.66, 64 x 3 (192 columns, one per
-// thread of kernel 4) 0.839 / 1.062.
+// a nu node in one register per lane (MU_S <= 32); 2, in two (MU_S 33 to 64);
+// 4, lines in shared memory.  The nodes win unless many lanes idle: kernel 4
+// packs a block's threads with columns of up to 4 rows, so that it is the
+// nodes' 32 / MU_S x MU_S lanes of 32 against its rows x W of 256.  With three
+// nodes nearly every column has clamped nu at both ends, three tasks in all.
+// 4 instances of 32 x 128 rows, MU_S x NU, kernel 4 / nodes, ms: 8 x 8 0.287 /
+// 0.244, 11 x 8 (22 lanes) 0.438 / 0.360, 19 x 8 0.768 / 0.672, 20 x 4 (20
+// lanes, W = 80) 0.364 / 0.391, 32 x 8 0.985 / 0.725, 32 x 3 0.434 / 0.487;
+// 33 x 8 1.84 / 1.31, 64 x 8 2.39 / 1.36, 64 x 4 1.018 / 0.803, 40 x 2 0.383 /
+// 0.367, 33 x 4 0.751 / 0.773, 33 x 5 0.834 / 0.918, 64 x 3 0.823 / 1.004.
 ATMO_HD int MultipleKind(const Shape& s) {
-  if (s.smus <= 32) return 32 / s.smus * s.smus >= 24 ? 1 : 4;
-  return s.smus <= 64 && s.sw() > 256 ? 2 : 4;
+  if (s.snu == 3) return 4;
+  if (s.smus <= 32) return 32 / s.smus * s.smus >= 22 || s.sw() > 128 ? 1 : 4;
+  return s.smus <= 64 && (s.sw() > 256 || (s.smus >= 40 && s.snu % 2 == 0)) ? 2 : 4;
 }
 
 // The scattering-density kernel of a LUT shape above order 2, a bit: arcs, 4
