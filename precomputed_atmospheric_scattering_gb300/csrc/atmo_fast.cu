@@ -1820,8 +1820,9 @@ cudaError_t LaunchMultipleFast(const Instance* insts, WorkList wl, int tiles, in
 // along the ray, and whose samples are in the planet's shadow together: a
 // shadowed sample reads nothing), a thread keeps its line columns of the last
 // two rows across samples, and two texel columns of a thread share a sample's
-// loads.  Per 16-instance launch at the reference's shape 3.55 -> 2.91 ms, one
-// high-resolution instance 2.74 -> 2.68 ms, one of half size 57 -> 47 us.
+// loads.  Per 16-instance launch at the reference's shape 3.55 -> 2.69 ms, one
+// high-resolution instance 2.74 -> 2.60 ms, one of half size 55 -> 35 us; over
+// shapes of 64 to 500 line columns and 24 to 1024 texel columns 0 to 45% less.
 // ---------------------------------------------------------------------------
 constexpr int kSingleSamples = kSingleScatteringSamples + 1;
 constexpr int kSingleThreads = 128;   // of a block of a shape of up to 256 columns
@@ -1976,6 +1977,15 @@ __device__ __forceinline__ void SingleFastBlock(const Instance& in, int local, f
   const uint32_t last = ((uint32_t)TW + (uint32_t)__float_as_int(magic)) * 12u;
   const int line_stride = G * R * line_floats;
   const int stages = (kSingleSamples + G - 1) / G;
+  // The block's threads build the lines of its rows side by side, line columns
+  // x_b, x_b + per_row, ... of row q_b each.  Where these are at most kBuild, a
+  // thread keeps those of the last even and the last odd LUT row in registers:
+  // of the rows around consecutive samples of a ray only 0.7 per sample are
+  // new at the reference's shape (predicated loads).
+  const int per_row = R == 1 ? threads : threads / R;
+  const int q_b = R == 1 ? 0 : (int)threadIdx.x / per_row;
+  const int x_b = R == 1 ? (int)threadIdx.x : (int)threadIdx.x - q_b * per_row;
+  const bool builds = q_b < R && row0 + q_b < rows_total && x_b < TW;
   int o0 = -1, o1 = -1;
   float4 ra[kBuild], rb[kBuild];
 #pragma unroll
@@ -1985,53 +1995,45 @@ __device__ __forceinline__ void SingleFastBlock(const Instance& in, int local, f
     const int first = stage * G;
     const int count = min(G, kSingleSamples - first);
     // The two transmittance LUT rows of each sample, interpolated in rho.
-    if (R == 1 && TW <= threads * kBuild) {
-      // One row per block, kBuild line columns per thread.  The thread keeps
-      // its columns of the last even and the last odd row in registers: of the
-      // rows around consecutive samples of a ray only 0.7 per sample are new
-      // at the reference's shape (predicated loads).
-      const int x = threadIdx.x, x_in = min(x, TW - 1);
-      if (row0 < rows_total) {
-        const float4* col = in.T + x_in;
-        float* out = buf + 3 * (x + 1);
-        const SunSample* srow = samp + first;
+    if (builds) {
+      const float4* col = in.T + x_b;
+      float* out = buf + q_b * line_floats + 3 * (x_b + 1);
+      const SunSample* srow = samp + q_b * kSingleSamples + first;
+      if (TW <= per_row * kBuild) {
         for (int g = 0; g < count; ++g) {
           const int4 v = *reinterpret_cast<const int4*>(&srow[g].t0);
           const float w0 = __int_as_float(v.z), w1 = __int_as_float(v.w);
 #pragma unroll
           for (int k = 0; k < kBuild; ++k) {
-            const int xk = k * threads;
-            const bool mine = x + xk < TW;
-            LoadIf(ra[k], ATMO_LINE_PTR(col, v.x, mine ? xk : 0, nT - x_in), mine && v.x != o0);
-            LoadIf(rb[k], ATMO_LINE_PTR(col, v.y, mine ? xk : 0, nT - x_in), mine && v.y != o1);
+            const bool mine = x_b + k * per_row < TW;
+            const int xk = mine ? k * per_row : 0;
+            LoadIf(ra[k], ATMO_LINE_PTR(col, v.x, xk, nT - x_b), mine && v.x != o0);
+            LoadIf(rb[k], ATMO_LINE_PTR(col, v.y, xk, nT - x_b), mine && v.y != o1);
           }
           o0 = v.x;
           o1 = v.y;
 #pragma unroll
           for (int k = 0; k < kBuild; ++k) {
-            if (x + k * threads < TW) {
-              out[3 * k * threads] = fmaf(w1, rb[k].x, w0 * ra[k].x);
-              out[3 * k * threads + 1] = fmaf(w1, rb[k].y, w0 * ra[k].y);
-              out[3 * k * threads + 2] = fmaf(w1, rb[k].z, w0 * ra[k].z);
+            if (x_b + k * per_row < TW) {
+              out[3 * k * per_row] = fmaf(w1, rb[k].x, w0 * ra[k].x);
+              out[3 * k * per_row + 1] = fmaf(w1, rb[k].y, w0 * ra[k].y);
+              out[3 * k * per_row + 2] = fmaf(w1, rb[k].z, w0 * ra[k].z);
             }
           }
-          out += line_floats;
+          out += R * line_floats;
         }
-      }
-    } else {
-      for (int g = 0; g < count; ++g) {
-        for (int q = 0; q < R; ++q) {
-          if (row0 + q >= rows_total) break;
-          const SunSample& sm = samp[q * kSingleSamples + first + g];
-          float* line_q = buf + (g * R + q) * line_floats;
-          for (int x = threadIdx.x; x < TW; x += threads) {
-            const float4 a = __ldg(ATMO_LINE_PTR(in.T, sm.t0, x, nT));
-            const float4 b = __ldg(ATMO_LINE_PTR(in.T, sm.t1, x, nT));
-            float* out = line_q + 3 * (x + 1);
-            out[0] = fmaf(sm.w1, b.x, sm.w0 * a.x);
-            out[1] = fmaf(sm.w1, b.y, sm.w0 * a.y);
-            out[2] = fmaf(sm.w1, b.z, sm.w0 * a.z);
+      } else {
+        for (int g = 0; g < count; ++g) {
+          const int4 v = *reinterpret_cast<const int4*>(&srow[g].t0);
+          const float w0 = __int_as_float(v.z), w1 = __int_as_float(v.w);
+          for (int x = 0; x_b + x < TW; x += per_row) {
+            const float4 a = __ldg(ATMO_LINE_PTR(col, v.x, x, nT - x_b));
+            const float4 b = __ldg(ATMO_LINE_PTR(col, v.y, x, nT - x_b));
+            out[3 * x] = fmaf(w1, b.x, w0 * a.x);
+            out[3 * x + 1] = fmaf(w1, b.y, w0 * a.y);
+            out[3 * x + 2] = fmaf(w1, b.z, w0 * a.z);
           }
+          out += R * line_floats;
         }
       }
     }
@@ -2086,21 +2088,30 @@ __device__ __forceinline__ void SingleFastBlock(const Instance& in, int local, f
   }
 }
 
-// A kernel per SingleKind, so that each has the registers it needs: one column
-// per thread up to 128 columns (64 registers), two up to 256 (72, 7 blocks of
-// 128 threads per SM; 6 blocks take 1% and 8 take 3% longer), four above (64, 4
-// blocks; 3 take 12% longer).
+// A kernel per SingleKind, so that each has the registers it needs.  Blocks per
+// SM: kSingleTwo 7 (72 registers; 6 take 1% and 8 take 3% longer),
+// kSingleTwoWide 4 (3 take 3% longer over 5 to 15 x 32 to 64 columns),
+// kSingleFour 3 (4 spill, and take 2 to 8% longer below 600 rows).
+ATMO_HD constexpr int SingleThreads(int kind) {
+  return kind == kSingleTwo ? kSingleThreads : kMultipleFastThreads;
+}
+ATMO_HD constexpr int SingleBlocks(int kind) {
+  return kind == kSingleTwo ? 7 : kind == kSingleFour ? 3 : 4;
+}
 template <int kKind>
-__global__ void __launch_bounds__(kKind == kSingleTwo ? kSingleThreads : kMultipleFastThreads,
-                                  kKind == kSingleTwo ? 7 : 4)
+__global__ void __launch_bounds__(SingleThreads(kKind), SingleBlocks(kKind))
 k_single_fast(const Instance* __restrict__ insts, WorkList wl, float magic) {
   extern __shared__ float4 smem[];
   int local;
   const Instance& in = insts[FindEntry(wl, blockIdx.x, &local)];
   if (SingleKind(in.s) != kKind) return;
-  if (kKind == kSingleOne) SingleFastBlock<1, 2, 0>(in, local, smem, magic);
-  if (kKind == kSingleTwo) SingleFastBlock<2, 2, kSingleThreads>(in, local, smem, magic);
-  if (kKind == kSingleFour) SingleFastBlock<4, 2, kMultipleFastThreads>(in, local, smem, magic);
+  constexpr int kThreads = kKind == kSingleOne ? 0 : SingleThreads(kKind);
+  constexpr int kCols = kKind == kSingleOne ? 1 : kKind == kSingleFour ? 4 : 2;
+  if (in.s.tw <= kThreads) {
+    SingleFastBlock<kCols, 1, kThreads>(in, local, smem, magic);
+  } else {
+    SingleFastBlock<kCols, 2, kThreads>(in, local, smem, magic);
+  }
 }
 
 cudaError_t LaunchSingleFast(const Instance* insts, WorkList wl, int tiles, int smem_bytes,
@@ -2111,12 +2122,16 @@ cudaError_t LaunchSingleFast(const Instance* insts, WorkList wl, int tiles, int 
     // Where every block of the launch is resident at once (4 per SM), threads
     // without a texel column help with the samples and the lines: one instance
     // of half size (1024 rows of 64 columns) 43 us against 51; 8 of them 260
-    // us against 234.
-    const int threads = tiles <= 4 * 152 ? kMultipleFastThreads : kSingleThreads;
-    k_single_fast<kSingleOne><<<tiles, threads, bytes, st>>>(insts, wl, kRoundMagic);
+    // us against 234.  Rows of more than 128 columns need them.
+    const bool all = tiles <= 4 * 152 || wl.kinds & kSingleOneWide;
+    k_single_fast<kSingleOne><<<tiles, all ? kMultipleFastThreads : kSingleThreads, bytes, st>>>(
+        insts, wl, kRoundMagic);
   }
   if (wl.kinds & kSingleTwo)
     k_single_fast<kSingleTwo><<<tiles, kSingleThreads, bytes, st>>>(insts, wl, kRoundMagic);
+  if (wl.kinds & kSingleTwoWide)
+    k_single_fast<kSingleTwoWide>
+        <<<tiles, kMultipleFastThreads, bytes, st>>>(insts, wl, kRoundMagic);
   if (wl.kinds & kSingleFour)
     k_single_fast<kSingleFour><<<tiles, kMultipleFastThreads, bytes, st>>>(insts, wl, kRoundMagic);
   return cudaGetLastError();

@@ -78,15 +78,21 @@ ATMO_HD int DensityKind(const Shape& s) {
 }
 // The single-scattering kernel of a LUT shape, a bit: one, two or four texel
 // columns of a row per thread.  Two share a sample's loads and hide each
-// other's latency; a row of up to 128 columns has one for every thread of a block (one
-// instance of 64 columns: 57 us with one per thread, 76 with two).
-constexpr int kSingleOne = 64, kSingleTwo = 128, kSingleFour = 256;
+// other's latency (256 columns, 16 instances: 2.97 ms against 3.20 with one);
+// a row of up to 128 columns has only one for each thread (64 columns, one
+// instance: 57 us, with two 76), and a row of wide transmittance lines, or of a
+// LUT of few rows, wants 256 threads to build the lines (204 columns, lines of
+// 339: 100 us against 150; 80 rows of 252 columns: 29 us against 31).
+constexpr int kSingleOne = 64, kSingleTwo = 128, kSingleTwoWide = 256, kSingleFour = 512;
+constexpr int kSingleOneWide = 1024;   // with kSingleOne: needs 256 threads
 ATMO_HD int SingleKind(const Shape& s) {
-  return s.sw() <= 128 ? kSingleOne : s.sw() <= 256 ? kSingleTwo : kSingleFour;
+  if (s.sw() <= 256)
+    return s.sw() <= 128 || s.tw > 256 || s.sr * s.smu < 304 ? kSingleOne : kSingleTwo;
+  return s.sw() <= 512 ? kSingleTwoWide : kSingleFour;
 }
-
 ATMO_HD int KernelKinds(const Shape& s) {
-  return MultipleKind(s) | DensityKind(s) | SingleKind(s);
+  return MultipleKind(s) | DensityKind(s) | SingleKind(s) |
+         (s.sw() > 128 && SingleKind(s) == kSingleOne ? kSingleOneWide : 0);
 }
 
 #ifdef __CUDACC__

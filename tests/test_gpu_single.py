@@ -37,3 +37,12 @@ def test_block_size_does_not_change_the_luts(atmo, oracle, torch):  # noqa: F811
     alone = scattering(1)[0]
     for many in scattering(48):   # 768 blocks, of 128 threads
         np.testing.assert_array_equal(many, alone)
+
+
+# Lines of two and more columns per thread beside several rows per block, rows
+# of one and of three columns per thread.
+@pytest.mark.parametrize("tw,mus,nu", [
+    (127, 7, 7), (200, 10, 3), (97, 16, 8), (258, 32, 8), (129, 40, 8), (257, 51, 13),
+    (400, 8, 3)])
+def test_line_columns_vs_oracle(atmo, oracle, torch, tw, mus, nu):  # noqa: F811
+    test_single_scattering_vs_oracle(atmo, oracle, torch, tw, mus, nu)
