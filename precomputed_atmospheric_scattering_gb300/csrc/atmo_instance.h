@@ -65,17 +65,23 @@ ATMO_HD int MultipleKind(const Shape& s) {
 
 // The scattering-density kernel of a LUT shape above order 2, a bit: arcs, 4
 // or 8 nu nodes per warp, or a table lookup per direction.  A warp of the arcs
-// is a long chain that needs blocks enough to fill the chip, and its work
-// grows with NU.  One instance, lookups / arcs, us: texels 57 k at NU 5 51 /
-// 43, 66 k at NU 4 51 / 39 and at NU 8 37 / 49, 131 k at NU 8 55 / 49, 262 k
-// at NU 16 104 / 102, 1 M at NU 8 301 / 182 (with 4 nodes per warp 219); 4 of
-// 2 M at NU 16 2258 / 1999.  Small LUTs take 4 nodes per warp: more warps.
+// is a long chain that needs blocks enough to fill the chip, slabs of (mu,
+// mu_s) texels; up to 12 nodes the groups of 8 have idle ones, unless they are
+// 5 to 8.  One and four instances, lookups / arcs of 4 / of 8, us, by slabs x
+// NU: 8192 x 8 35 / 51 / 68 and 98 / 68 / 68; 12288 x 3 47 / 37 / 43, x 6 51 /
+// 45 / 59 and 137 / 104 / 80, x 9 90 / 53 / 72 and 209 / 137 / 184, x 14 102 /
+// 94 / 94 and 266 / 236 / 260; 16384 x 8 53 / 51 / 68 and 182 / 127 / 98;
+// 24576 x 8 96 / 68 / 68 and 252 / 174 / 172; 32768 x 9 154 / 127 / 107 and 471
+// / 342 / 354, x 14 190 / 178 / 148 and 632 / 585 / 503; 131072 x 8 281 / 225 /
+// 184 and 1058 / 800 / 606, x 12 426 / 404 / 442 and 1603 / 1519 / 1582.
 constexpr int kDensityArcs4 = 8, kDensityArcs8 = 16, kDensityLookups = 32;
 ATMO_HD int DensityKind(const Shape& s) {
-  const long long texels = s.s_texels();
-  if (s.snu > 16 || s.iw > 512 || texels < (s.snu <= 5 ? 49152 : 131072)) return kDensityLookups;
-  return s.snu <= 4 || texels < 262144 ? kDensityArcs4 : kDensityArcs8;
+  const long long slabs = (long long)s.sr * s.smu * s.smus;
+  if (s.snu > 16 || s.iw > 512 || slabs < 12288) return kDensityLookups;
+  if (s.snu <= 4 || (s.snu > 8 && s.snu <= 12)) return kDensityArcs4;
+  return slabs > 16384 ? kDensityArcs8 : kDensityArcs4;
 }
+
 // The single-scattering kernel of a LUT shape, a bit: one, two or four texel
 // columns of a row per thread.  Two share a sample's loads and hide each
 // other's latency (256 columns, 16 instances: 2.97 ms against 3.20 with one);
