@@ -79,7 +79,8 @@ ATMO_HD int DensityKind(const Shape& s) {
   const long long slabs = (long long)s.sr * s.smu * s.smus;
   if (s.snu > 16 || s.iw > 512 || slabs < 12288) return kDensityLookups;
   if (s.snu <= 4 || (s.snu > 8 && s.snu <= 12)) return kDensityArcs4;
-  return slabs > 16384 ? kDensityArcs8 : kDensityArcs4;
+  if (slabs > 16384) return kDensityArcs8;
+  return s.snu <= 8 ? kDensityArcs4 : kDensityLookups;
 }
 
 // The single-scattering kernel of a LUT shape, a bit: one, two or four texel
