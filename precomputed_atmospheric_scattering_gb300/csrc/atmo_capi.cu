@@ -648,46 +648,41 @@ atmo_status atmo_precompute(const atmo_atmosphere* atmosphere, const atmo_lut_sh
   in.I = reinterpret_cast<float4*>(irradiance);
   in.combined = combined ? 1 : 0;
   in.blend = blend ? 1 : 0;
-  // Temporaries, stream ordered.
+  // Temporaries and launch descriptors: one stream-ordered allocation.
+  Program prog;
+  prog.path = path;
+  prog.slots.push_back(in);
+  prog.orders.push_back(num_scattering_orders);
+  prog.AddStage({0});
   const size_t nT = (size_t)s.t_texels();
-  const size_t bytes[9] = {nI * 16, nS * 16, nS * 16, nS * 16,
-                           (size_t)s.sr * s.smu * sizeof(TexelRow),
-                           (size_t)s.smus * sizeof(TexelCol),
-                           (size_t)s.sr * kDensityThetaSamples * sizeof(DensityRow),
-                           (size_t)s.ih * sizeof(IrrRow) + (size_t)s.iw * sizeof(float),
-                           nT * 16};
-  void* tmp[9] = {nullptr};
-  for (int i = 0; i < 9; ++i) {
-    cudaError_t e = cudaMallocAsync(&tmp[i], bytes[i], st);
-    if (e != cudaSuccess) {
-      for (int j = 0; j < i; ++j) cudaFreeAsync(tmp[j], st);
-      return CudaFail(e, "cudaMallocAsync");
-    }
-  }
-  in.dI = (float4*)tmp[0];
-  in.dR = (float4*)tmp[1];
-  in.dM = (float4*)tmp[2];
-  in.dJ = (float4*)tmp[3];
-  in.tab.rows = (TexelRow*)tmp[4];
-  in.tab.cols = (TexelCol*)tmp[5];
-  in.tab.drows = (DensityRow*)tmp[6];
-  in.tab.irows = (IrrRow*)tmp[7];
-  in.tab.mus_i = (float*)((char*)tmp[7] + (size_t)s.ih * sizeof(IrrRow));
-  in.Tau = (float4*)tmp[8];
-  atmo_status result;
-  {
-    Program prog;
-    prog.path = path;
-    prog.slots.push_back(in);
-    prog.orders.push_back(num_scattering_orders);
-    prog.AddStage({0});
-    result = prog.Run(st, /*use_graph=*/false);
-    // The program's work lists are freed when it goes out of scope: wait for
-    // the launches that read them.
-    cudaError_t e = cudaStreamSynchronize(st);
-    if (result == ATMO_OK && e != cudaSuccess) result = CudaFail(e, "precompute");
-  }
-  for (int i = 0; i < 9; ++i) cudaFreeAsync(tmp[i], st);
+  const size_t bytes[11] = {nI * 16, nS * 16, nS * 16, nS * 16, nT * 16,
+                            (size_t)s.sr * s.smu * sizeof(TexelRow),
+                            (size_t)s.smus * sizeof(TexelCol),
+                            (size_t)s.sr * kDensityThetaSamples * sizeof(DensityRow),
+                            (size_t)s.ih * sizeof(IrrRow), (size_t)s.iw * sizeof(float),
+                            prog.DescriptorBytes()};
+  size_t at[12] = {0};
+  for (int i = 0; i < 11; ++i) at[i + 1] = at[i] + (bytes[i] + 255) / 256 * 256;
+  char* tmp = nullptr;
+  const cudaError_t ae = cudaMallocAsync(&tmp, at[11], st);
+  if (ae != cudaSuccess) return CudaFail(ae, "cudaMallocAsync");
+  Instance& slot = prog.slots[0];
+  slot.dI = (float4*)(tmp + at[0]);
+  slot.dR = (float4*)(tmp + at[1]);
+  slot.dM = (float4*)(tmp + at[2]);
+  slot.dJ = (float4*)(tmp + at[3]);
+  slot.Tau = (float4*)(tmp + at[4]);
+  slot.tab.rows = (TexelRow*)(tmp + at[5]);
+  slot.tab.cols = (TexelCol*)(tmp + at[6]);
+  slot.tab.drows = (DensityRow*)(tmp + at[7]);
+  slot.tab.irows = (IrrRow*)(tmp + at[8]);
+  slot.tab.mus_i = (float*)(tmp + at[9]);
+  prog.PlaceDescriptors(tmp + at[10]);
+  atmo_status result = prog.Run(st, /*use_graph=*/false);
+  // The LUTs are complete when the call returns.
+  const cudaError_t e = cudaStreamSynchronize(st);
+  if (result == ATMO_OK && e != cudaSuccess) result = CudaFail(e, "precompute");
+  cudaFreeAsync(tmp, st);
   return result;
 }
 

@@ -76,19 +76,14 @@ atmo_status Storage::Allocate(const Shape& shape, bool combined_textures, bool h
   half = half_precision;
   const size_t nT = (size_t)s.t_texels(), nI = (size_t)s.i_texels(),
                nS = (size_t)s.s_texels();
-  auto alloc = [&](void** p, size_t bytes) -> atmo_status {
-    cudaError_t e = cudaMalloc(p, bytes);
-    if (e != cudaSuccess) {
-      *p = nullptr;
-      Free();
-      return CudaFail(e, "cudaMalloc");
-    }
-    owned.push_back(*p);
-    return ATMO_OK;
+  // One allocation, each buffer on a 256-byte boundary: first the offsets.
+  std::vector<std::pair<void**, size_t>> parts;
+  size_t total = 0;
+  auto place = [&](void** p, size_t bytes) {
+    parts.push_back({p, total});
+    total += (bytes + 255) / 256 * 256;
   };
-  atmo_status st;
-#define ATMO_ALLOC(ptr, bytes)                                   \
-  if ((st = alloc(reinterpret_cast<void**>(&(ptr)), (bytes))) != ATMO_OK) return st;
+#define ATMO_ALLOC(ptr, bytes) place(reinterpret_cast<void**>(&(ptr)), (bytes))
   ATMO_ALLOC(T, nT * sizeof(float4));
   ATMO_ALLOC(Tau, nT * sizeof(float4));
   ATMO_ALLOC(I, nI * sizeof(float4));
@@ -110,6 +105,14 @@ atmo_status Storage::Allocate(const Shape& shape, bool combined_textures, bool h
   ATMO_ALLOC(tab.mus_i, (size_t)s.iw * sizeof(float));
   if (UsesRowOrder(s)) ATMO_ALLOC(tab.row_order, (size_t)s.sr * s.smu * sizeof(int));
 #undef ATMO_ALLOC
+  char* base = nullptr;
+  const cudaError_t e = cudaMalloc(&base, total);
+  if (e != cudaSuccess) {
+    Free();
+    return CudaFail(e, "cudaMalloc");
+  }
+  owned.push_back(base);
+  for (const auto& part : parts) *part.first = base + part.second;
   return ATMO_OK;
 }
 
@@ -219,9 +222,8 @@ Program::~Program() {
   if (ev_fork_) cudaEventDestroy(ev_fork_);
   if (ev_join_) cudaEventDestroy(ev_join_);
   if (upload_done_) cudaEventDestroy(upload_done_);
-  if (d_slots_) cudaFree(d_slots_);
-  if (h_slots_pinned_) cudaFreeHost(h_slots_pinned_);
-  if (d_blob_) cudaFree(d_blob_);
+  if (owns_descriptors_) cudaFree(d_slots_);
+  if (h_pinned_) cudaFreeHost(h_pinned_);
 }
 
 int Program::AddWorkList(const std::vector<int>& members, Pass pass, int order, int* tiles,
@@ -292,25 +294,39 @@ void Program::AddToHalf(const std::vector<int>& members) {
   }
 }
 
+// The descriptors reach the device as by-value parameters of up to three
+// launches where they fit: no pinned staging buffer to allocate (0.1 ms and
+// more of a program that runs once), and no copy engine between the stream's
+// kernels.  More of them are copied from a pinned buffer.
+constexpr int kDescriptorWords = 1000, kMaxWordLaunches = 3;
+struct DescriptorWords {
+  int count;
+  int w[kDescriptorWords];
+};
+__global__ void k_write_descriptors(const __grid_constant__ DescriptorWords d, int* dst) {
+  for (int i = threadIdx.x; i < d.count; i += blockDim.x) dst[i] = d.w[i];
+}
+static_assert(sizeof(Instance) % sizeof(int) == 0, "descriptors are copied as words");
+
 atmo_status Program::Finalize() {
   if (finalized_) return ATMO_OK;
-  if (!blob_.empty()) {
-    ATMO_CUDA_TRY(cudaMalloc(&d_blob_, blob_.size() * sizeof(int)));
-    ATMO_CUDA_TRY(cudaMemcpy(d_blob_, blob_.data(), blob_.size() * sizeof(int),
-                             cudaMemcpyHostToDevice));
+  if (!d_slots_) {
+    ATMO_CUDA_TRY(cudaMalloc(&d_slots_, DescriptorBytes()));
+    owns_descriptors_ = true;
   }
+  const int* lists = reinterpret_cast<const int*>(d_slots_ + slots.size());
   wls_.clear();
   for (auto& o : wl_offsets_) {
     WorkList w;
-    w.inst = d_blob_ + o.first;
-    w.start = d_blob_ + o.first + o.second;
+    w.inst = lists + o.first;
+    w.start = lists + o.first + o.second;
     w.count = o.second;
     w.kinds = 0;
     for (int i = 0; i < o.second; ++i) w.kinds |= KernelKinds(slots[blob_[o.first + i]].s);
     wls_.push_back(w);
   }
-  ATMO_CUDA_TRY(cudaMalloc(&d_slots_, slots.size() * sizeof(Instance)));
-  ATMO_CUDA_TRY(cudaMallocHost(&h_slots_pinned_, slots.size() * sizeof(Instance)));
+  if (DescriptorBytes() > kMaxWordLaunches * kDescriptorWords * sizeof(int))
+    ATMO_CUDA_TRY(cudaMallocHost(&h_pinned_, DescriptorBytes()));
   // Row orders of the instances that have the table (slots of one model share
   // it; the radii of a later set_atmosphere leave the order stale, which
   // changes nothing in the LUTs).
@@ -332,15 +348,30 @@ atmo_status Program::Finalize() {
 }
 
 atmo_status Program::Upload(cudaStream_t st) {
+  const size_t slot_words = slots.size() * sizeof(Instance) / sizeof(int);
+  words_.resize(slot_words + blob_.size());
+  std::memcpy(words_.data(), slots.data(), slot_words * sizeof(int));
+  std::copy(blob_.begin(), blob_.end(), words_.begin() + slot_words);
+  if (!h_pinned_) {
+    int* dst = reinterpret_cast<int*>(d_slots_);
+    for (size_t i = 0; i < words_.size(); i += kDescriptorWords) {
+      DescriptorWords d;
+      d.count = (int)std::min(words_.size() - i, (size_t)kDescriptorWords);
+      std::memcpy(d.w, words_.data() + i, d.count * sizeof(int));
+      k_write_descriptors<<<1, 256, 0, st>>>(d, dst + i);
+    }
+    ATMO_CUDA_TRY(cudaGetLastError());
+    return ATMO_OK;
+  }
   if (!upload_done_) {
     ATMO_CUDA_TRY(cudaEventCreateWithFlags(&upload_done_, cudaEventDisableTiming));
   } else {
     // The previous run's copy may still be reading the staging buffer.
     ATMO_CUDA_TRY(cudaEventSynchronize(upload_done_));
   }
-  std::memcpy(h_slots_pinned_, slots.data(), slots.size() * sizeof(Instance));
-  ATMO_CUDA_TRY(cudaMemcpyAsync(d_slots_, h_slots_pinned_, slots.size() * sizeof(Instance),
-                                cudaMemcpyHostToDevice, st));
+  std::memcpy(h_pinned_, words_.data(), DescriptorBytes());
+  ATMO_CUDA_TRY(cudaMemcpyAsync(d_slots_, h_pinned_, DescriptorBytes(), cudaMemcpyHostToDevice,
+                                st));
   ATMO_CUDA_TRY(cudaEventRecord(upload_done_, st));
   return ATMO_OK;
 }
@@ -468,7 +499,19 @@ atmo_status Program::Run(cudaStream_t st, bool use_graph) {
   atmo_status s = Finalize();
   if (s != ATMO_OK) return s;
   if ((s = Upload(st)) != ATMO_OK) return s;
-  if (!use_graph) return Launch(st);
+  // A first run launches its kernels one by one: a program that runs once (a
+  // model initialised once) would pay 0.1 ms and more for a graph it replays
+  // once.  Into a capturing stream it goes by the graph, which is refused.
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  if (!launched_ && (cudaStreamIsCapturing(st, &capturing) != cudaSuccess ||
+                     capturing != cudaStreamCaptureStatusNone)) {
+    cudaGetLastError();
+    launched_ = true;
+  }
+  if (!use_graph || !launched_) {
+    launched_ = true;
+    return Launch(st);
+  }
   if (!graph_) {
     if (!capture_stream_) {
       ATMO_CUDA_TRY(cudaStreamCreateWithFlags(&capture_stream_, cudaStreamNonBlocking));

@@ -38,7 +38,7 @@ struct Storage {
          *dR = nullptr, *dM = nullptr, *dJ = nullptr, *S = nullptr, *M = nullptr;
   void *S_half = nullptr, *M_half = nullptr;   // half-precision outputs
   Tables tab{};
-  std::vector<void*> owned;                    // what Free() releases
+  std::vector<void*> owned;                    // what Free() releases (one allocation)
   atmo_status Allocate(const Shape& shape, bool combined_textures, bool half_precision);
   void Free();
   size_t Bytes() const;
@@ -70,13 +70,21 @@ class Program {
   void AddStage(const std::vector<int>& members, bool transmittance_only = false);
   // Appends the FP32 -> FP16 conversion of the slots' scattering outputs.
   void AddToHalf(const std::vector<int>& members);
-  atmo_status Finalize();              // uploads work lists
-  atmo_status Upload(cudaStream_t st); // copies slots to the device
+  // Bytes of the launch descriptors (slots and work lists) on the device.
+  size_t DescriptorBytes() const {
+    return slots.size() * sizeof(Instance) + blob_.size() * sizeof(int);
+  }
+  // Has the program keep its descriptors in the caller's device memory of at
+  // least DescriptorBytes() (before the first run).
+  void PlaceDescriptors(void* device) { d_slots_ = static_cast<Instance*>(device); }
+  atmo_status Finalize();              // places the descriptors
+  atmo_status Upload(cudaStream_t st); // copies the descriptors to the device
   atmo_status Launch(cudaStream_t st); // enqueues the steps
   atmo_status LaunchStep(size_t i, cudaStream_t st);
   // Runs the steps without a graph, timing each with CUDA events on `st`.
   atmo_status TimeSteps(cudaStream_t st, std::vector<float>* ms);
-  // Upload + replay through a CUDA graph (captured on first use).
+  // Upload + launch; with use_graph, the second and later runs replay a CUDA
+  // graph.
   atmo_status Run(cudaStream_t st, bool use_graph);
   int KernelCount() const { return (int)steps_.size(); }
   std::vector<Step> const& steps() const { return steps_; }
@@ -88,9 +96,11 @@ class Program {
   std::vector<int> blob_;              // inst[] then start[] of every work list
   std::vector<std::pair<int, int>> wl_offsets_;  // (offset, count)
   std::vector<WorkList> wls_;
-  Instance* d_slots_ = nullptr;
-  Instance* h_slots_pinned_ = nullptr;
-  int* d_blob_ = nullptr;
+  Instance* d_slots_ = nullptr;        // the slots, then the work lists
+  bool owns_descriptors_ = false;
+  std::vector<int> words_;             // host copy of what d_slots_ points to
+  void* h_pinned_ = nullptr;           // staging copy of many slots
+  bool launched_ = false;
   cudaGraphExec_t graph_ = nullptr;
   cudaStream_t capture_stream_ = nullptr;
   cudaEvent_t upload_done_ = nullptr;    // guards reuse of the pinned staging copy
