@@ -89,8 +89,8 @@ ATMO_HD float4 to4(F3 a, float w) { return make_float4(a.x, a.y, a.z, w); }
 // rescaling: 2 instructions for 6): lengths, cosines and their quotients, where
 // a subnormal stands for zero.  Transmittances and radiances keep div_approx
 // and the division operator.
-ATMO_HD float quot(float a, float b) {
-#if defined(__CUDA_ARCH__) && defined(ATMO_FLUSHED_GEOMETRY)
+ATMO_HD float QuotFlushed(float a, float b) {
+#ifdef __CUDA_ARCH__
   float y;
   asm("div.approx.ftz.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b));
   return y;
@@ -98,8 +98,8 @@ ATMO_HD float quot(float a, float b) {
   return a / b;
 #endif
 }
-ATMO_HD float root(float x) {
-#if defined(__CUDA_ARCH__) && defined(ATMO_FLUSHED_GEOMETRY)
+ATMO_HD float RootFlushed(float x) {
+#ifdef __CUDA_ARCH__
   float y;
   asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
@@ -107,6 +107,13 @@ ATMO_HD float root(float x) {
   return sqrtf(x);
 #endif
 }
+#ifdef ATMO_FLUSHED_GEOMETRY
+ATMO_HD float quot(float a, float b) { return QuotFlushed(a, b); }
+ATMO_HD float root(float x) { return RootFlushed(x); }
+#else
+ATMO_HD float quot(float a, float b) { return a / b; }
+ATMO_HD float root(float x) { return sqrtf(x); }
+#endif
 
 ATMO_HD float clampf(float x, float lo, float hi) { return fminf(fmaxf(x, lo), hi); }
 // GLSL smoothstep; for the degenerate e0 == e1 (a point sun) it returns 0 at

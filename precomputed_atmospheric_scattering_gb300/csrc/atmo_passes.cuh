@@ -122,21 +122,30 @@ ATMO_PASS float ProfileDensity64(const ProfileF& p, double h) {
 
 // ProfileDensity for the optical-length samples: a layer without an
 // exponential term (the ozone layers) skips its exp (its product with 0).
-ATMO_PASS float SampleDensity(const ProfileF& p, float h) {
-  const LayerF& l = h < p.layer[0].width ? p.layer[0] : p.layer[1];
-  const float e = l.exp_term == 0.0f ? 0.0f : l.exp_term * expf(l.exp_scale * h);
-  return clampf(e + l.linear_term * h + l.constant_term, 0.0f, 1.0f);
+ATMO_PASS float SampleDensity(const LayerF& l0, const LayerF& l1, float h) {
+  const bool low = h < l0.width;
+  const float term = low ? l0.exp_term : l1.exp_term, scale = low ? l0.exp_scale : l1.exp_scale;
+  const float e = term == 0.0f ? 0.0f : term * expf(scale * h);
+  return clampf(e + (low ? l0.linear_term : l1.linear_term) * h +
+                    (low ? l0.constant_term : l1.constant_term),
+                0.0f, 1.0f);
 }
 
+// The layers are read once and selected from registers, and a sample's
+// altitude takes the approximate square root and quotient (<= 2 ulp; the LUT's
+// error against 64 bits is the same: rms 1.0e-6 over 8 atmospheres and sizes).
 ATMO_PASS void OpticalLengthPartial(const Consts& c, const TransmittanceRay& ray, int first,
                                     int stride, float out[3]) {
   Kahan kr, km, ka;
-  const float near_ground = 1e-5f * (c.Rt - c.Rb);
+  const float near_ground = 1e-5f * (c.Rt - c.Rb), rb = c.Rb, rb2 = c.Rb * c.Rb, h2 = c.H * c.H;
+  const LayerF r0 = c.prof_r.layer[0], r1 = c.prof_r.layer[1], m0 = c.prof_m.layer[0],
+               m1 = c.prof_m.layer[1], a0 = c.prof_a.layer[0], a1 = c.prof_a.layer[1];
   for (int q = first; q <= kOpticalLengthSamples; q += stride) {
-    float d = float(q) * ray.dx;
-    RadialPoint p = PointAlongRay(c, ray.rho, ray.rmu, d);
+    const float d = float(q) * ray.dx;
+    const float rho2 = clampf(fmaf(d, d + 2.0f * ray.rmu, ray.rho * ray.rho), 0.0f, h2);
+    const float h = QuotFlushed(rho2, RootFlushed(rho2 + rb2) + rb);
     float w = (q == 0 || q == kOpticalLengthSamples) ? 0.5f : 1.0f;
-    if (ray.horizon && p.h < near_ground) {
+    if (ray.horizon && h < near_ground) {
       // A sample at the tangent point of a horizon ray: the reference's
       // unclamped FP64 altitude decides between the layers (it can be
       // slightly negative, selecting layer 0).
@@ -149,9 +158,9 @@ ATMO_PASS void OpticalLengthPartial(const Consts& c, const TransmittanceRay& ray
       ka.add(ProfileDensity64(c.prof_a, h) * w);
       continue;
     }
-    kr.add(SampleDensity(c.prof_r, p.h) * w);
-    km.add(SampleDensity(c.prof_m, p.h) * w);
-    ka.add(SampleDensity(c.prof_a, p.h) * w);
+    kr.add(SampleDensity(r0, r1, h) * w);
+    km.add(SampleDensity(m0, m1, h) * w);
+    ka.add(SampleDensity(a0, a1, h) * w);
   }
   out[0] = kr.s;
   out[1] = km.s;
