@@ -330,9 +330,9 @@ atmo_status Program::Finalize() {
   // Row orders of the instances that have the table (slots of one model share
   // it; the radii of a later set_atmosphere leave the order stale, which
   // changes nothing in the LUTs).
-  fork_indirect_ = !slots.empty();
+  fork_ = !slots.empty();
   for (const Instance& in : slots)
-    if (!in.dI2 || in.dI2 == in.dI) fork_indirect_ = false;
+    if (!in.dI2 || in.dI2 == in.dI) fork_ = false;
   std::vector<int*> done;
   for (const Instance& in : slots) {
     if (!in.tab.row_order ||
@@ -377,7 +377,7 @@ atmo_status Program::Upload(cudaStream_t st) {
 }
 
 atmo_status Program::PrepareFork() {
-  if (!fork_indirect_ || side_stream_) return ATMO_OK;
+  if (!fork_ || side_stream_) return ATMO_OK;
   ATMO_CUDA_TRY(cudaStreamCreateWithFlags(&side_stream_, cudaStreamNonBlocking));
   ATMO_CUDA_TRY(cudaEventCreateWithFlags(&ev_fork_, cudaEventDisableTiming));
   ATMO_CUDA_TRY(cudaEventCreateWithFlags(&ev_join_, cudaEventDisableTiming));
@@ -386,23 +386,35 @@ atmo_status Program::PrepareFork() {
 
 atmo_status Program::Launch(cudaStream_t st) {
   for (size_t i = 0; i < steps_.size(); ++i) {
-    // The indirect irradiance of order n - 1 runs beside the density pass of
-    // order n: they write and read different delta-irradiance buffers and
-    // both only read the previous order's scattering, which the multiple
-    // scattering of order n overwrites after joining both.  The indirect
-    // pass's small grid then fills the density launch's gaps.
-    if (fork_indirect_ && steps_[i].pass == Pass::kDensity && i + 1 < steps_.size() &&
-        steps_[i + 1].pass == Pass::kIndirect && steps_[i + 1].order == steps_[i].order - 1) {
-      atmo_status s = PrepareFork();
-      if (s != ATMO_OK) return s;
-      ATMO_CUDA_TRY(cudaEventRecord(ev_fork_, st));
-      ATMO_CUDA_TRY(cudaStreamWaitEvent(side_stream_, ev_fork_, 0));
-      if ((s = LaunchStep(i + 1, side_stream_)) != ATMO_OK) return s;
-      ATMO_CUDA_TRY(cudaEventRecord(ev_join_, side_stream_));
-      if ((s = LaunchStep(i, st)) != ATMO_OK) return s;
-      ATMO_CUDA_TRY(cudaStreamWaitEvent(st, ev_join_, 0));
-      ++i;
-      continue;
+    // Pairs of passes that run side by side, the smaller one on the side
+    // stream, where it fills the other's gaps:
+    // the set-up tables beside the transmittance, which does not read them
+    // (the tables are one long FP64 chain on a few SMs);
+    // the direct irradiance and the density rows' ground transmittance beside
+    // single scattering, which reads neither;
+    // the indirect irradiance of order n - 1 beside the density pass of order
+    // n: they write and read different delta-irradiance buffers and both only
+    // read the previous order's scattering, which the multiple scattering of
+    // order n overwrites after joining both.
+    if (fork_ && i + 1 < steps_.size()) {
+      const Pass first = steps_[i].pass, second = steps_[i + 1].pass;
+      const bool pair = (first == Pass::kTables && second == Pass::kTransmittance) ||
+                        (first == Pass::kDirect && second == Pass::kSingle);
+      const bool indirect = first == Pass::kDensity && second == Pass::kIndirect &&
+                            steps_[i + 1].order == steps_[i].order - 1;
+      if (pair || indirect) {
+        const size_t side = pair ? i : i + 1, main = pair ? i + 1 : i;
+        atmo_status s = PrepareFork();
+        if (s != ATMO_OK) return s;
+        ATMO_CUDA_TRY(cudaEventRecord(ev_fork_, st));
+        ATMO_CUDA_TRY(cudaStreamWaitEvent(side_stream_, ev_fork_, 0));
+        if ((s = LaunchStep(side, side_stream_)) != ATMO_OK) return s;
+        ATMO_CUDA_TRY(cudaEventRecord(ev_join_, side_stream_));
+        if ((s = LaunchStep(main, st)) != ATMO_OK) return s;
+        ATMO_CUDA_TRY(cudaStreamWaitEvent(st, ev_join_, 0));
+        ++i;
+        continue;
+      }
     }
     atmo_status s = LaunchStep(i, st);
     if (s != ATMO_OK) return s;

@@ -105,9 +105,9 @@ class Program {
   cudaStream_t capture_stream_ = nullptr;
   cudaEvent_t upload_done_ = nullptr;    // guards reuse of the pinned staging copy
   bool finalized_ = false;
-  // Indirect irradiance beside density (every slot has two delta-irradiance
-  // buffers): the side stream and the fork / join events of Launch.
-  bool fork_indirect_ = false;
+  // Passes side by side (every slot has two delta-irradiance buffers): the
+  // side stream and the fork / join events of Launch.
+  bool fork_ = false;
   atmo_status PrepareFork();             // creates the side stream and events once
   cudaStream_t side_stream_ = nullptr;
   cudaEvent_t ev_fork_ = nullptr, ev_join_ = nullptr;
