@@ -301,6 +301,29 @@ bool DensityFastFits(const Shape& s) { return DensityBaseSmem(s, 2) <= 48 * 1024
 template <bool kOrder2>
 __host__ __device__ constexpr int DensityTexelsPerTask() { return 4; }
 
+// A block's tasks (a mu row and up to 4 of its texels each) go to its threads
+// in rounds of 256.  The tasks of the last round, where they are at most half
+// as many (in whole warps), are split into parts of the 16 theta rows, whose
+// sums are added in order through shared memory: a slab of half the
+// reference's size has 64 tasks, which kept 2 of a block's 8 warps busy (order
+// 2, one such instance 86 -> 49 us, 8 of them 545 -> 293; 70 shapes of 16
+// to 250 mu rows and 3 to 15 nodes: 19% less time).
+__host__ __device__ inline int DensityTasks(const Shape& s) { return s.smu * ((s.snu + 3) / 4); }
+__host__ __device__ inline int DensityLastRound(const Shape& s) {
+  return DensityTasks(s) % kDensityFastThreads;
+}
+__host__ __device__ inline int DensityParts(const Shape& s, int order) {
+  const int last = DensityLastRound(s), warps = (last + 31) / 32;
+  if (last == 0 || warps > kDensityFastThreads / 64) return 1;
+  const int parts = kDensityFastThreads / 32 / warps;
+  return DensityBaseSmem(s, order) + parts * last * 4 * (int)sizeof(F3) <= 48 * 1024 ? parts : 1;
+}
+// The parts' sums, bytes (a multiple of 16).
+__host__ __device__ inline int DensityPartSmem(const Shape& s, int order) {
+  const int parts = DensityParts(s, order);
+  return parts > 1 ? parts * DensityLastRound(s) * 4 * (int)sizeof(F3) : 0;
+}
+
 // The outgoing direction's phase functions and the scattering coefficients
 // fold into one weight per channel and direction, shared by the task's 4
 // texels (one mu row: one altitude), so a texel keeps one sum.
@@ -466,9 +489,12 @@ k_density_fast(const Instance* __restrict__ insts, WorkList wl, int order, int s
   float4* E = smem;                                            // [16][NU + 1] entries
   float4* G = E + kDensityThetaSamples * row_entries * (kStride / 16);
   float4* V = G + (s.iw + 1) * (kNodeBytes / 16);              // [species][16][NU], [IW] values
+  constexpr int kSmemOrder = kOrder2 ? 2 : 3;
+  F3* part_sums = reinterpret_cast<F3*>(V + kSpecies * nodes + s.iw);
   // Above order 2: the merge rows, their table layout (offset, J, j0, size in
   // entries; size 0 when not merged) and the merged tables.
-  MergeRow* meta = reinterpret_cast<MergeRow*>(V + kSpecies * nodes + s.iw);
+  MergeRow* meta = reinterpret_cast<MergeRow*>(V + kSpecies * nodes + s.iw +
+                                               DensityPartSmem(s, kSmemOrder) / 16);
   int4* build = reinterpret_cast<int4*>(meta + kDensityThetaSamples);
   int& merged_entries = *reinterpret_cast<int*>(build + kDensityThetaSamples);
   float4* X = reinterpret_cast<float4*>(build + kDensityThetaSamples + 1);
@@ -535,7 +561,8 @@ k_density_fast(const Instance* __restrict__ insts, WorkList wl, int order, int s
   if (!kOrder2 && threadIdx.x == 0) {
     // Table offsets, rows in theta order while they fit the budget.
     // The budget: the launch's shared memory beyond this instance's tables.
-    const int budget = max(smem_bytes - DensityBaseSmem(s, 3), 0) / kNodeBytes;
+    const int budget =
+        max(smem_bytes - DensityBaseSmem(s, 3) - DensityPartSmem(s, 3), 0) / kNodeBytes;
     const uint32_t xbase = (uint32_t)__cvta_generic_to_shared(X);
     int off = 0;
     for (int l = 0; l < kDensityThetaSamples; ++l) {
@@ -630,9 +657,13 @@ k_density_fast(const Instance* __restrict__ insts, WorkList wl, int order, int s
   const float dtdp = (kPiF / 16.0f) * (kPiF / 16.0f);
   const uint32_t e_base = (uint32_t)__cvta_generic_to_shared(E);
   const uint32_t ir_adj = RowAdjust((uint32_t)__cvta_generic_to_shared(G), kNodeBytes, magic);
-  const int per_row = (NU + kDensityTexelsPerTask - 1) / kDensityTexelsPerTask;
-  const int tasks = s.smu * per_row;
-  for (int ti = threadIdx.x; ti < tasks; ti += blockDim.x) {
+  const int tasks = DensityTasks(s), last = DensityLastRound(s);
+  const int parts_last = DensityParts(s, kSmemOrder);
+  for (int first = 0; first < tasks; first += kDensityFastThreads) {
+    const int parts = tasks - first == last ? parts_last : 1;
+    const int part = parts > 1 ? (int)threadIdx.x / ((last + 31) & ~31) : 0;
+    const int id = (int)threadIdx.x - part * ((last + 31) & ~31), ti = first + id;
+    if (part >= parts || ti >= tasks) break;
     const int j = ti % s.smu, n0 = (ti / s.smu) * kDensityTexelsPerTask;
     const TexelRow row = in.tab.rows[k * s.smu + j];
     DensityTask<kOrder2> task;
@@ -649,7 +680,8 @@ k_density_fast(const Instance* __restrict__ insts, WorkList wl, int order, int s
     // Order 2: the ground point's mu_g = (r mu_s + dist nu1) / Rb; its
     // irradiance coordinate 1/2 + kg mu_g is w0 + kg dist nu1 / Rb.
     const float w0 = fmaf(row.r * cc.mu_s * inv_rb, kg, 0.5f);
-    for (int l = 0; l < kDensityThetaSamples; ++l) {
+    const int l_end = (part + 1) * kDensityThetaSamples / parts;
+    for (int l = part * kDensityThetaSamples / parts; l < l_end; ++l) {
       const DensityRow dr = drows[l];
       const float B = row.mu * dr.cos_t;
       const float oxs = row.omega_x * dr.sin_t;
@@ -699,11 +731,23 @@ k_density_fast(const Instance* __restrict__ insts, WorkList wl, int order, int s
     }
 #pragma unroll
     for (int q = 0; q < kDensityTexelsPerTask; ++q) {
-      if (n0 + q < NU) {
-        const F3 J = ToF3(task.sum[q]);
+      const F3 J = ToF3(task.sum[q]);
+      if (parts > 1) {
+        part_sums[(part * last + id) * kDensityTexelsPerTask + q] = J;
+      } else if (n0 + q < NU) {
         in.dJ[(k * s.smu + j) * W + (n0 + q) * s.smus + col] = to4(J, 1.0f);
       }
     }
+  }
+  if (parts_last == 1) return;
+  __syncthreads();
+  for (int e = threadIdx.x; e < last * kDensityTexelsPerTask; e += kDensityFastThreads) {
+    const int ti = tasks - last + e / kDensityTexelsPerTask;
+    const int j = ti % s.smu, n = ti / s.smu * kDensityTexelsPerTask + e % kDensityTexelsPerTask;
+    F3 J = part_sums[e];
+    for (int part = 1; part < parts_last; ++part)
+      J += part_sums[part * last * kDensityTexelsPerTask + e];
+    if (n < NU) in.dJ[(k * s.smu + j) * W + n * s.smus + col] = to4(J, 1.0f);
   }
 }
 
@@ -778,7 +822,7 @@ __host__ __device__ inline int DensityArcSmem(const Shape& s) {
 }
 
 int DensityFastSmem(const Shape& s, const Consts& c, int order) {
-  const int base = DensityBaseSmem(s, order);
+  const int base = DensityBaseSmem(s, order) + DensityPartSmem(s, order);
   if (order == 2) return base;
   if (DensityKind(s) != kDensityLookups) return DensityArcSmem(s);
   const int room = kDensityMaxSmem - base;

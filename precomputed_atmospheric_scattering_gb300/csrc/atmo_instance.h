@@ -66,21 +66,23 @@ ATMO_HD int MultipleKind(const Shape& s) {
 // The scattering-density kernel of a LUT shape above order 2, a bit: arcs, 4
 // or 8 nu nodes per warp, or a table lookup per direction.  A warp of the arcs
 // is a long chain that needs blocks enough to fill the chip, slabs of (mu,
-// mu_s) texels; up to 12 nodes the groups of 8 have idle ones, unless they are
-// 5 to 8.  One and four instances, lookups / arcs of 4 / of 8, us, by slabs x
-// NU: 8192 x 8 35 / 51 / 68 and 98 / 68 / 68; 12288 x 3 47 / 37 / 43, x 6 51 /
-// 45 / 59 and 137 / 104 / 80, x 9 90 / 53 / 72 and 209 / 137 / 184, x 14 102 /
-// 94 / 94 and 266 / 236 / 260; 16384 x 8 53 / 51 / 68 and 182 / 127 / 98;
-// 24576 x 8 96 / 68 / 68 and 252 / 174 / 172; 32768 x 9 154 / 127 / 107 and 471
-// / 342 / 354, x 14 190 / 178 / 148 and 632 / 585 / 503; 131072 x 8 281 / 225 /
-// 184 and 1058 / 800 / 606, x 12 426 / 404 / 442 and 1603 / 1519 / 1582.
+// mu_s) texels; its lanes are 32 mu rows, of which some idle in the last group
+// of an odd MU; and up to 12 nodes the groups of 8 have idle ones, unless they
+// are 5 to 8.  One and four instances, lookups / arcs of 4 / of 8, us, by
+// slabs x NU: 8192 x 8 35 / 51 / 68 and 96 / 68 / 68; 12288 x 3 47 / 37 / 43, x
+// 6 51 / 45 / 59 and 137 / 104 / 80, x 9 90 / 53 / 72 and 209 / 137 / 184;
+// 16384 x 8 53 / 51 / 68 and 162 / 127 / 98, x 14 102 / 94 / 94 and 328 / 320 /
+// 285; 24576 x 8 96 / 68 / 68 and 252 / 174 / 172; 32768 x 9 154 / 127 / 107
+// and 471 / 342 / 354, x 14 190 / 178 / 148 and 632 / 585 / 503; 131072 x 8 281
+// / 225 / 184 and 1058 / 800 / 606; MU = 100 (100 lanes of 128): 51200 x 12
+// four 705 / 768 / 809, x 16 279 / 340 / 311 and 924 / 1234 / 1026.
 constexpr int kDensityArcs4 = 8, kDensityArcs8 = 16, kDensityLookups = 32;
 ATMO_HD int DensityKind(const Shape& s) {
   const long long slabs = (long long)s.sr * s.smu * s.smus;
   if (s.snu > 16 || s.iw > 512 || slabs < 12288) return kDensityLookups;
+  if (s.snu > 10 && 8 * s.smu < 7 * ((s.smu + 31) / 32 * 32)) return kDensityLookups;
   if (s.snu <= 4 || (s.snu > 8 && s.snu <= 12)) return kDensityArcs4;
-  if (slabs > 16384) return kDensityArcs8;
-  return s.snu <= 8 ? kDensityArcs4 : kDensityLookups;
+  return s.snu > 12 || slabs > 16384 ? kDensityArcs8 : kDensityArcs4;
 }
 
 // The single-scattering kernel of a LUT shape, a bit: one, two or four texel
