@@ -121,6 +121,10 @@ __device__ __forceinline__ int FindEntry(const WorkList& wl, int tile, int* loca
 constexpr int kTransmittanceLanes = 16;                 // lanes per texel
 constexpr int kTransmittanceThreads = 256;
 constexpr int kTransmittanceTexelsPerTile = kTransmittanceThreads / kTransmittanceLanes;
+constexpr int kHorizonTexelsPerTile = 32 / kTransmittanceLanes;   // one warp's
+ATMO_HD int HorizonTiles(const Shape& s) {
+  return (s.th + kHorizonTexelsPerTile - 1) / kHorizonTexelsPerTile;
+}
 constexpr int kTexelThreads = 128;                      // per-texel kernels
 constexpr int kIndirectThreads = 128;                   // one warp per texel
 constexpr int kIndirectTexelsPerTile = kIndirectThreads / 32;

@@ -10,22 +10,41 @@ namespace atmo {
 
 // Transmittance: kTransmittanceLanes lanes per texel split the 501 samples of
 // each optical length; the partial Kahan sums are reduced with shuffles.
-// Bound by instruction issue; 64 registers (4 blocks per SM): per 16-instance
+//
+// Bound by instruction issue; 64 registers (4 blocks per SM; 92 and 48 take
+// longer).  The horizon column's FP64 rays, a chain of 5 us, are a warp's in
+// the first blocks and not in every row's last block, whose other threads
+// waited for it at the end.  Per 16-instance
 // launch at the reference's shape 0.568 -> 0.458 ms with the layers in
-// registers and the approximate altitude of OpticalLengthPartial, 0.525 at 92
-// registers, 0.566 at 48.
+// registers and the approximate altitude of OpticalLengthPartial -> 0.415; one
+// instance 49 -> 42 -> 35 us.
 __global__ void __launch_bounds__(kTransmittanceThreads, 4)
 k_transmittance(const Instance* __restrict__ insts, WorkList wl) {
+  __shared__ HorizonRay horizon[kHorizonTexelsPerTile];
   int local;
   const Instance& in = insts[FindEntry(wl, blockIdx.x, &local)];
-  const int lane = threadIdx.x % kTransmittanceLanes;
-  const int texel = local * kTransmittanceTexelsPerTile + threadIdx.x / kTransmittanceLanes;
-  const bool valid = texel < in.s.t_texels();
+  const int lane = threadIdx.x % kTransmittanceLanes, slot = threadIdx.x / kTransmittanceLanes;
+  // The first warps of the first blocks take the horizon column's texels.
+  const int tw = in.s.tw, th = in.s.th, with = HorizonTiles(in.s);
+  const bool is_horizon = local < with && slot < kHorizonTexelsPerTile;
+  int i = tw - 1, j = local * kHorizonTexelsPerTile + slot;
+  if (is_horizon) {
+    if (lane == 0 && j < th) horizon[slot] = MakeHorizonRay(in.c, in.s, j);
+    __syncwarp();
+  } else {
+    const int e = local * kTransmittanceTexelsPerTile + slot -
+                  min(local + 1, with) * kHorizonTexelsPerTile;
+    i = e % (tw - 1);
+    j = e / (tw - 1);
+  }
+  const int texel = j * tw + i;
+  const bool valid = j < th;
   float sums[3] = {0.0f, 0.0f, 0.0f};
   TransmittanceRay ray{0.0f, 0.0f, 0.0f};
   if (valid) {
-    ray = TransmittanceTexelRay(in.c, in.s, texel);
-    OpticalLengthPartial(in.c, ray, lane, kTransmittanceLanes, sums);
+    ray = TransmittanceTexelRay(in.c, in.s, i, j);
+    OpticalLengthPartial(in.c, ray, is_horizon ? horizon + slot : nullptr, lane,
+                         kTransmittanceLanes, sums);
   }
 #pragma unroll
   for (int off = kTransmittanceLanes / 2; off > 0; off >>= 1) {
@@ -187,6 +206,16 @@ k_indirect_irradiance(const Instance* __restrict__ insts, WorkList wl, int order
 // ---------------------------------------------------------------------------
 // Host-side launchers.
 // ---------------------------------------------------------------------------
+int TransmittanceTiles(const Shape& s) {
+  const long long others = s.t_texels() - s.th;   // besides the horizon column's
+  const int with = HorizonTiles(s);
+  const long long left =
+      others - (long long)with * (kTransmittanceTexelsPerTile - kHorizonTexelsPerTile);
+  return with + (left > 0 ? (int)((left + kTransmittanceTexelsPerTile - 1) /
+                                  kTransmittanceTexelsPerTile)
+                          : 0);
+}
+
 cudaError_t LaunchTransmittance(const Instance* insts, WorkList wl, int tiles, cudaStream_t st) {
   k_transmittance<<<tiles, kTransmittanceThreads, 0, st>>>(insts, wl);
   return cudaGetLastError();

@@ -10,6 +10,7 @@ namespace atmo {
 
 int TableTiles(const Shape& s);
 cudaError_t LaunchTables(const Instance* insts, WorkList wl, int tiles, cudaStream_t st);
+int TransmittanceTiles(const Shape& s);
 cudaError_t LaunchTransmittance(const Instance* insts, WorkList wl, int tiles, cudaStream_t st);
 cudaError_t LaunchDirectIrradiance(const Instance* insts, WorkList wl, int tiles,
                                    cudaStream_t st);

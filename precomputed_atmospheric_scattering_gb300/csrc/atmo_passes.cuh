@@ -8,8 +8,10 @@
 
 #ifdef __CUDACC__
 #define ATMO_PASS __device__ __forceinline__
+#define ATMO_PASS_COLD static __device__ __noinline__
 #else
 #define ATMO_PASS inline
+#define ATMO_PASS_COLD inline
 #define __constant__
 #endif
 #include "atmo_trig.inc"
@@ -23,11 +25,6 @@ namespace atmo {
 // ---------------------------------------------------------------------------
 struct TransmittanceRay {
   float rho, rmu, dx;
-  // The reference's own FP64 ray (functions.glsl:275-299 after :427-448) for
-  // the horizon column, whose tangent ray can dip below the ground by FP64
-  // rounding; zero elsewhere.
-  double r64, rmu64_2, dx64;
-  bool horizon;
 };
 
 // IEEE double operations that are never contracted into FMAs, so that the
@@ -62,8 +59,7 @@ ATMO_PASS double dsqrt(double a) {
 #endif
 }
 
-ATMO_PASS TransmittanceRay TransmittanceTexelRay(const Consts& c, const Shape& s, int texel) {
-  int i = texel % s.tw, j = texel / s.tw;
+ATMO_PASS TransmittanceRay TransmittanceTexelRay(const Consts& c, const Shape& s, int i, int j) {
   // GetRMuFromTransmittanceTextureUv at the texel centre: x = i / (n - 1).
   float x_mu = float(i) / float(s.tw - 1);
   float x_r = float(j) / float(s.th - 1);
@@ -78,30 +74,33 @@ ATMO_PASS TransmittanceRay TransmittanceTexelRay(const Consts& c, const Shape& s
   // r mu = (H^2 - rho^2 - d^2) / (2 d); mu = 1 when d = 0.
   ray.rmu = d == 0.0f ? r : clampf((hm - d * d) / (2.0f * d), -r, r);
   ray.dx = d / float(kOpticalLengthSamples);
-  ray.horizon = i == s.tw - 1;
-  ray.r64 = ray.rmu64_2 = ray.dx64 = 0.0;
-  if (ray.horizon) {
-    // functions.glsl:427-448, :207-214, :285-289 in the reference's order.
-    const double Rb = c.dRb, Rt = c.dRt;
-    double u = ddiv(double(i) + 0.5, double(s.tw)), v = ddiv(double(j) + 0.5, double(s.th));
-    double xm = ddiv(dsub(u, ddiv(0.5, double(s.tw))), dsub(1.0, ddiv(1.0, double(s.tw))));
-    double xr = ddiv(dsub(v, ddiv(0.5, double(s.th))), dsub(1.0, ddiv(1.0, double(s.th))));
-    double H = dsqrt(dsub(dmul(Rt, Rt), dmul(Rb, Rb)));
-    double rh = dmul(H, xr);
-    double rr = dsqrt(dadd(dmul(rh, rh), dmul(Rb, Rb)));
-    double dmn = dsub(Rt, rr), dmx = dadd(rh, H);
-    double dd = dadd(dmn, dmul(xm, dsub(dmx, dmn)));
-    double mu = dd == 0.0 ? 1.0
-                          : ddiv(dsub(dsub(dmul(H, H), dmul(rh, rh)), dmul(dd, dd)),
-                                 dmul(dmul(2.0, rr), dd));
-    mu = fmin(fmax(mu, -1.0), 1.0);
-    double disc = dadd(dmul(dmul(rr, rr), dsub(dmul(mu, mu), 1.0)), dmul(Rt, Rt));
-    double dist = fmax(dadd(-dmul(rr, mu), dsqrt(fmax(disc, 0.0))), 0.0);
-    ray.r64 = rr;
-    ray.rmu64_2 = dmul(dmul(2.0, rr), mu);
-    ray.dx64 = ddiv(dist, double(kOpticalLengthSamples));
-  }
   return ray;
+}
+
+// The reference's own FP64 ray (functions.glsl:275-299 after :427-448) for the
+// horizon column's texel of row j: its tangent ray can dip below the ground by
+// FP64 rounding.
+struct HorizonRay {
+  double r, rmu_2, dx;
+};
+ATMO_PASS HorizonRay MakeHorizonRay(const Consts& c, const Shape& s, int j) {
+  // functions.glsl:427-448, :207-214, :285-289 in the reference's order.
+  const double Rb = c.dRb, Rt = c.dRt;
+  double u = ddiv(double(s.tw - 1) + 0.5, double(s.tw)), v = ddiv(double(j) + 0.5, double(s.th));
+  double xm = ddiv(dsub(u, ddiv(0.5, double(s.tw))), dsub(1.0, ddiv(1.0, double(s.tw))));
+  double xr = ddiv(dsub(v, ddiv(0.5, double(s.th))), dsub(1.0, ddiv(1.0, double(s.th))));
+  double H = dsqrt(dsub(dmul(Rt, Rt), dmul(Rb, Rb)));
+  double rh = dmul(H, xr);
+  double rr = dsqrt(dadd(dmul(rh, rh), dmul(Rb, Rb)));
+  double dmn = dsub(Rt, rr), dmx = dadd(rh, H);
+  double dd = dadd(dmn, dmul(xm, dsub(dmx, dmn)));
+  double mu = dd == 0.0 ? 1.0
+                        : ddiv(dsub(dsub(dmul(H, H), dmul(rh, rh)), dmul(dd, dd)),
+                               dmul(dmul(2.0, rr), dd));
+  mu = fmin(fmax(mu, -1.0), 1.0);
+  double disc = dadd(dmul(dmul(rr, rr), dsub(dmul(mu, mu), 1.0)), dmul(Rt, Rt));
+  double dist = fmax(dadd(-dmul(rr, mu), dsqrt(fmax(disc, 0.0))), 0.0);
+  return HorizonRay{rr, dmul(dmul(2.0, rr), mu), ddiv(dist, double(kOpticalLengthSamples))};
 }
 
 struct Kahan {
@@ -131,11 +130,25 @@ ATMO_PASS float SampleDensity(const LayerF& l0, const LayerF& l1, float h) {
                 0.0f, 1.0f);
 }
 
+// The three densities at sample q, near the tangent point of a horizon ray: the
+// reference's unclamped FP64 altitude decides between the layers (it can be
+// slightly negative, selecting layer 0).  Out of line: one to three samples of
+// a texel, whose registers the loop would pay for.
+ATMO_PASS_COLD F3 TangentDensities(const Consts& c, const HorizonRay& ray, int q) {
+  const double di = dmul(double(q), ray.dx);
+  const double ri = dsqrt(dadd(dadd(dmul(di, di), dmul(ray.rmu_2, di)), dmul(ray.r, ray.r)));
+  const double h = dsub(ri, c.dRb);
+  return F3{ProfileDensity64(c.prof_r, h), ProfileDensity64(c.prof_m, h),
+            ProfileDensity64(c.prof_a, h)};
+}
+
 // The layers are read once and selected from registers, and a sample's
 // altitude takes the approximate square root and quotient (<= 2 ulp; the LUT's
 // error against 64 bits is the same: rms 1.0e-6 over 8 atmospheres and sizes).
-ATMO_PASS void OpticalLengthPartial(const Consts& c, const TransmittanceRay& ray, int first,
-                                    int stride, float out[3]) {
+// horizon: the texel's FP64 ray in the horizon column, else null.
+ATMO_PASS void OpticalLengthPartial(const Consts& c, const TransmittanceRay& ray,
+                                    const HorizonRay* horizon, int first, int stride,
+                                    float out[3]) {
   Kahan kr, km, ka;
   const float near_ground = 1e-5f * (c.Rt - c.Rb), rb = c.Rb, rb2 = c.Rb * c.Rb, h2 = c.H * c.H;
   const LayerF r0 = c.prof_r.layer[0], r1 = c.prof_r.layer[1], m0 = c.prof_m.layer[0],
@@ -145,17 +158,11 @@ ATMO_PASS void OpticalLengthPartial(const Consts& c, const TransmittanceRay& ray
     const float rho2 = clampf(fmaf(d, d + 2.0f * ray.rmu, ray.rho * ray.rho), 0.0f, h2);
     const float h = QuotFlushed(rho2, RootFlushed(rho2 + rb2) + rb);
     float w = (q == 0 || q == kOpticalLengthSamples) ? 0.5f : 1.0f;
-    if (ray.horizon && h < near_ground) {
-      // A sample at the tangent point of a horizon ray: the reference's
-      // unclamped FP64 altitude decides between the layers (it can be
-      // slightly negative, selecting layer 0).
-      double di = dmul(double(q), ray.dx64);
-      double ri = dsqrt(dadd(dadd(dmul(di, di), dmul(ray.rmu64_2, di)),
-                             dmul(ray.r64, ray.r64)));
-      double h = dsub(ri, c.dRb);
-      kr.add(ProfileDensity64(c.prof_r, h) * w);
-      km.add(ProfileDensity64(c.prof_m, h) * w);
-      ka.add(ProfileDensity64(c.prof_a, h) * w);
+    if (horizon && h < near_ground) {
+      const F3 density = TangentDensities(c, *horizon, q);
+      kr.add(density.x * w);
+      km.add(density.y * w);
+      ka.add(density.z * w);
       continue;
     }
     kr.add(SampleDensity(r0, r1, h) * w);

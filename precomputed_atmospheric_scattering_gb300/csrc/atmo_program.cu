@@ -201,7 +201,7 @@ int Tiles(Pass pass, const Shape& s, atmo_path path, int order) {
   auto cdiv = [](long long a, long long b) { return (int)((a + b - 1) / b); };
   switch (pass) {
     case Pass::kTables: return TableTiles(s);
-    case Pass::kTransmittance: return cdiv(s.t_texels(), kTransmittanceTexelsPerTile);
+    case Pass::kTransmittance: return TransmittanceTiles(s);
     case Pass::kDirect: return cdiv(s.i_texels() + s.sr * kDensityThetaSamples, kTexelThreads);
     case Pass::kSingle:
       return path == ATMO_PATH_FAST ? SingleFastTiles(s) : cdiv(s.s_texels(), kTexelThreads);
