@@ -16,7 +16,7 @@ namespace atmo {
 // the first blocks and not in every row's last block, whose other threads
 // waited for it at the end.  Per 16-instance
 // launch at the reference's shape 0.568 -> 0.458 ms with the layers in
-// registers and the approximate altitude of OpticalLengthPartial -> 0.415; one
+// registers and the approximate altitude of OpticalLengthPartial -> 0.426; one
 // instance 49 -> 42 -> 35 us.
 __global__ void __launch_bounds__(kTransmittanceThreads, 4)
 k_transmittance(const Instance* __restrict__ insts, WorkList wl) {

@@ -142,9 +142,18 @@ ATMO_PASS_COLD F3 TangentDensities(const Consts& c, const HorizonRay& ray, int q
             ProfileDensity64(c.prof_a, h)};
 }
 
-// The layers are read once and selected from registers, and a sample's
-// altitude takes the approximate square root and quotient (<= 2 ulp; the LUT's
-// error against 64 bits is the same: rms 1.0e-6 over 8 atmospheres and sizes).
+// A sample's altitude a / b, b in [2 Rb, 2 Rt]: the approximate reciprocal's
+// product, corrected by its residual (Newton's step for a quotient).
+ATMO_PASS float SampleAltitude(float a, float b) {
+  const float y = QuotFlushed(1.0f, b), h = a * y;
+  return fmaf(fmaf(-h, b, a), y, h);
+}
+
+// The layers are read once and selected from registers, and a sample's radius
+// takes the approximate square root (its error is halved in the altitude).  The
+// LUT's error against 64 bits, mean over 40 atmospheres and sizes, relative: rms
+// 1.0191e-6 (1.0192e-6 with IEEE forms), mean 3.063e-7 (3.066e-7), of the norm
+// 9.42e-8 (9.40e-8); an uncorrected quotient 1.0202e-6, 3.075e-7, 9.51e-8.
 // horizon: the texel's FP64 ray in the horizon column, else null.
 ATMO_PASS void OpticalLengthPartial(const Consts& c, const TransmittanceRay& ray,
                                     const HorizonRay* horizon, int first, int stride,
@@ -156,7 +165,7 @@ ATMO_PASS void OpticalLengthPartial(const Consts& c, const TransmittanceRay& ray
   for (int q = first; q <= kOpticalLengthSamples; q += stride) {
     const float d = float(q) * ray.dx;
     const float rho2 = clampf(fmaf(d, d + 2.0f * ray.rmu, ray.rho * ray.rho), 0.0f, h2);
-    const float h = QuotFlushed(rho2, RootFlushed(rho2 + rb2) + rb);
+    const float h = SampleAltitude(rho2, RootFlushed(rho2 + rb2) + rb);
     float w = (q == 0 || q == kOpticalLengthSamples) ? 0.5f : 1.0f;
     if (horizon && h < near_ground) {
       const F3 density = TangentDensities(c, *horizon, q);
