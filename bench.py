@@ -66,18 +66,18 @@ METRIC = "Earth LUT rebuilds/s batched vs plain on 1 GB300 @<=1e-3 vs FP64; p99 
 UNIT = "rebuilds/s"
 WORKLOAD = ("Earth LUT rebuild, 256x64/256x128x32/64x16 RGBA FP32, 4 orders, 3 wavelengths, "
             "combined")
-# FP32 operations per direction sample that the fast scattering-density kernel
-# executes, from ncu's SASS op counters over one launch (an FMA counts 2, a
+# FP32 operations per direction sample that the fast scattering-density kernels
+# execute, from ncu's opcode counters over one launch (an FMA counts 2, a
 # packed FP32x2 instruction 2 or 4): order 2 evaluates single scattering with
-# its phase functions, higher orders one radiance table (one merged sky +
-# ground table on the rows that hit the ground).
-DENSITY_FLOPS_PER_SAMPLE = {2: 48.9, 3: 20.1}
+# its phase functions at every direction, higher orders sum the directions of a
+# theta row by arcs (prefix sums of the phase functions).
+DENSITY_FLOPS_PER_SAMPLE = {2: 44.3, 3: 5.4}
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one density
 # launch over 16 default-shape Earth instances, from a one-pass ncu capture of
 # the batch-16 rebuild (python -m precomputed_atmospheric_scattering_gb300.
-# profile_case --batch 16): order 2 read 67.8 MB + wrote 207.4 MB, orders 3
-# and 4 read 36.0 MB + wrote 207.5 MB.
-DENSITY_DRAM_BYTES_B16 = {2: 275.27e6, 3: 243.53e6}
+# profile_case --batch 16): order 2 read 67.8 MB + wrote 206.9 MB, orders 3
+# and 4 read 35.8 MB + wrote 207.8 MB.
+DENSITY_DRAM_BYTES_B16 = {2: 274.72e6, 3: 243.62e6}
 # Bytes a density launch must move per default-shape Earth instance: the
 # previous order's mu rows that its 16 theta samples interpolate (484 unique
 # rows of the 4,096 per instance, 1.98 MB per species; two species at order
@@ -513,7 +513,7 @@ def roofline_entry(batch, B, peak, stream, rebuilds_per_s):
     compulsory = sum(DENSITY_COMPULSORY_BYTES[min(o, 3)] * B for o, _ in dens) / len(dens)
     hbm, _ = hbm_peak()
     launch_s = dens_ms / len(dens) * 1e-3
-    roof = {"bound": "fp32", "kernel": "k_density_fast",
+    roof = {"bound": "fp32", "kernel": "k_density_fast<1>, k_density_arcs<8>",
             "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
             "peak_source": "measured FP32 FMA rate",
             "traffic": traffic, "compulsory_bytes": compulsory,
