@@ -655,16 +655,16 @@ atmo_status atmo_precompute(const atmo_atmosphere* atmosphere, const atmo_lut_sh
   prog.orders.push_back(num_scattering_orders);
   prog.AddStage({0});
   const size_t nT = (size_t)s.t_texels();
-  const size_t bytes[11] = {nI * 16, nS * 16, nS * 16, nS * 16, nT * 16,
+  const size_t bytes[12] = {nI * 16, nS * 16, nS * 16, nS * 16, nT * 16,
                             (size_t)s.sr * s.smu * sizeof(TexelRow),
                             (size_t)s.smus * sizeof(TexelCol),
                             (size_t)s.sr * kDensityThetaSamples * sizeof(DensityRow),
                             (size_t)s.ih * sizeof(IrrRow), (size_t)s.iw * sizeof(float),
-                            prog.DescriptorBytes()};
-  size_t at[12] = {0};
-  for (int i = 0; i < 11; ++i) at[i + 1] = at[i] + (bytes[i] + 255) / 256 * 256;
+                            prog.DescriptorBytes(), nI * 16};
+  size_t at[13] = {0};
+  for (int i = 0; i < 12; ++i) at[i + 1] = at[i] + (bytes[i] + 255) / 256 * 256;
   char* tmp = nullptr;
-  const cudaError_t ae = cudaMallocAsync(&tmp, at[11], st);
+  const cudaError_t ae = cudaMallocAsync(&tmp, at[12], st);
   if (ae != cudaSuccess) return CudaFail(ae, "cudaMallocAsync");
   Instance& slot = prog.slots[0];
   slot.dI = (float4*)(tmp + at[0]);
@@ -678,6 +678,7 @@ atmo_status atmo_precompute(const atmo_atmosphere* atmosphere, const atmo_lut_sh
   slot.tab.irows = (IrrRow*)(tmp + at[8]);
   slot.tab.mus_i = (float*)(tmp + at[9]);
   prog.PlaceDescriptors(tmp + at[10]);
+  slot.dI2 = (float4*)(tmp + at[11]);   // two buffers: passes side by side
   atmo_status result = prog.Run(st, /*use_graph=*/false);
   // The LUTs are complete when the call returns.
   const cudaError_t e = cudaStreamSynchronize(st);
