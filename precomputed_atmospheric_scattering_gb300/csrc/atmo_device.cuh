@@ -487,6 +487,15 @@ ATMO_HD Lookup4 MakeLookup(const Shape& s, float u_nu, float u_mu_s, float u_mu,
 }
 
 ATMO_HD int ClampIdx(int i, int n) { return i < 0 ? 0 : (i > n - 1 ? n - 1 : i); }
+// A float as the device converts it to an int, truncated and saturated, NaN to
+// 0 (undefined on a host where the value does not fit).
+ATMO_HD int ToInt(float x) {
+#ifndef __CUDA_ARCH__
+  if (!(x >= -2147483648.0f)) return x != x ? 0 : INT32_MIN;
+  if (x >= 2147483648.0f) return INT32_MAX;
+#endif
+  return (int)x;
+}
 
 // The 4D lookup of functions.glsl:958-976: two trilinear fetches (the nu
 // nodes' blocks b0 and b1) that share their y (mu) and z (r) interpolation, with
@@ -531,6 +540,34 @@ ATMO_HD F3 Scattering4(const float4* __restrict__ tex, const Shape& s, const Loo
              t6.z * v6 + t7.z * v7;
   }
   return acc;
+}
+
+// The texels of a lookup that two lanes make together (ScatteringPairs): the
+// texel row of the lower mu row and r slice, and in one word the lower node's
+// first column (x 4) and whether the upper mu row (1) and r slice (2) are
+// others.
+struct PairLookup {
+  int row, code;
+};
+ATMO_HD PairLookup MakePairLookup(const Shape& s, const Lookup4& L) {
+  const int W = s.sw(), Hh = s.smu, D = s.sr;
+  const int y = ToInt(floorf(L.y)), z = ToInt(floorf(L.z)), x = ToInt(floorf(L.xl));
+  // A ray that misses the atmosphere has any z, up to the largest int, whose
+  // successor is the smallest: a step where the next slice is in the LUT.
+  const int step_y = y >= 0 && y < Hh - 1, step_z = z >= 0 && z < D - 1;
+  PairLookup p;
+  p.row = (ClampIdx(z, D) * Hh + ClampIdx(y, Hh)) * W;
+  p.code = (ClampIdx(L.b0 + x + 1, W + 1) - 1) * 4 + step_y + 2 * step_z;
+  return p;
+}
+// The texel row of the lower (0) or upper mu row (1) and r slice (2).
+ATMO_HD int PairRow(const Shape& s, const PairLookup& p, int upper) {
+  const int step = p.code & upper;
+  return p.row + (step & 1) * s.sw() + (step >> 1) * s.smu * s.sw();
+}
+// The lower (0) or upper (1) mu_s column of nu node 0 or 1.
+ATMO_HD int PairColumn(const Shape& s, const PairLookup& p, int node, int upper) {
+  return ClampIdx((p.code >> 2) + node * s.smus + upper, s.sw());
 }
 
 // functions.glsl:739-747

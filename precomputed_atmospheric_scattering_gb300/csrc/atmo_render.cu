@@ -98,34 +98,29 @@ __device__ float4 ScatteringRGBA(const float4* __restrict__ tex, const Shape& s,
 // its neighbours.
 __device__ float4 ScatteringPairs(const float4* __restrict__ tex, const Shape& s,
                                   const Lookup4& L) {
-  const int W = s.sw(), Hh = s.smu, D = s.sr;
+  [[maybe_unused]] const int texels = s.sw() * s.smu * s.sr;   // checked build
   const int lane = threadIdx.x & 31, odd = lane & 1;
-  const float fy = floorf(L.y), fz = floorf(L.z), fx = floorf(L.xl);
-  const float b = L.y - fy, c = L.z - fz, a = L.xl - fx;
-  const int j0 = ClampIdx((int)fy, Hh), j1 = ClampIdx((int)fy + 1, Hh);
-  const int k0 = ClampIdx((int)fz, D), k1 = ClampIdx((int)fz + 1, D);
-  const int row = (k0 * Hh + j0) * W;
-  const int col = (ClampIdx(L.b0 + (int)fx + 1, W + 1) - 1) * 4 + (j1 - j0) + 2 * (k1 - k0);
+  const float b = L.y - floorf(L.y), c = L.z - floorf(L.z), a = L.xl - floorf(L.xl);
+  const PairLookup own = MakePairLookup(s, L);
   float4 out = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
   for (int round = 0; round < 2; ++round) {
     const int src = (lane & ~1) | round;
-    const int r = __shfl_sync(0xffffffffu, row, src), x = __shfl_sync(0xffffffffu, col, src);
+    const PairLookup p{__shfl_sync(0xffffffffu, own.row, src),
+                       __shfl_sync(0xffffffffu, own.code, src)};
     const float qa = __shfl_sync(0xffffffffu, a, src), qb = __shfl_sync(0xffffffffu, b, src);
     const float qc = __shfl_sync(0xffffffffu, c, src);
     const float l1 = __shfl_sync(0xffffffffu, L.lerp_nu, src);
-    const int dj = (x & 1) * W, dk = (x >> 1 & 1) * Hh * W;
     const float wx = odd ? qa : 1.0f - qa;
-    const int rows[4] = {r, r + dj, r + dk, r + dj + dk};
     const float wr[4] = {(1.0f - qb) * (1.0f - qc), qb * (1.0f - qc), (1.0f - qb) * qc, qb * qc};
     float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
     for (int node = 0; node < 2; ++node) {
-      const int i = ClampIdx((x >> 2) + node * s.smus + odd, W);
+      const int i = PairColumn(s, p, node, odd);
       const float wn = wx * (node == 0 ? 1.0f - l1 : l1);
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        const float4 t = __ldg(ATMO_CHECKED_PTR(kCheckLutTexel, tex, rows[q], i, W * Hh * D));
+        const float4 t = __ldg(ATMO_CHECKED_PTR(kCheckLutTexel, tex, PairRow(s, p, q), i, texels));
         const float w = wn * wr[q];
         acc.x = fmaf(t.x, w, acc.x);
         acc.y = fmaf(t.y, w, acc.y);
