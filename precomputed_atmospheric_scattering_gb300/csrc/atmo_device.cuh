@@ -557,13 +557,21 @@ ATMO_HD PairLookup MakePairLookup(const Shape& s, const Lookup4& L) {
   const int step_y = y >= 0 && y < Hh - 1, step_z = z >= 0 && z < D - 1;
   PairLookup p;
   p.row = (ClampIdx(z, D) * Hh + ClampIdx(y, Hh)) * W;
-  p.code = (ClampIdx(L.b0 + x + 1, W + 1) - 1) * 4 + step_y + 2 * step_z;
+  // Bounded so that the word holds it, but below column 0 by a node and more:
+  // nu below -1 by rounding has the lower node's columns there, and the upper
+  // node's (all of the weight) MU_S above them.
+  const int col = ClampIdx(L.b0 + x + s.smus + 1, W + s.smus + 1) - s.smus - 1;
+  p.code = col * 4 + step_y + 2 * step_z;
   return p;
 }
-// The texel row of the lower (0) or upper mu row (1) and r slice (2).
-ATMO_HD int PairRow(const Shape& s, const PairLookup& p, int upper) {
-  const int step = p.code & upper;
-  return p.row + (step & 1) * s.sw() + (step >> 1) * s.smu * s.sw();
+// The texel rows of the lower mu row and r slice, the upper mu row, the upper
+// slice, and both.
+ATMO_HD void PairRows(const Shape& s, const PairLookup& p, int rows[4]) {
+  const int dj = (p.code & 1) * s.sw(), dk = (p.code >> 1 & 1) * s.smu * s.sw();
+  rows[0] = p.row;
+  rows[1] = p.row + dj;
+  rows[2] = p.row + dk;
+  rows[3] = p.row + dj + dk;
 }
 // The lower (0) or upper (1) mu_s column of nu node 0 or 1.
 ATMO_HD int PairColumn(const Shape& s, const PairLookup& p, int node, int upper) {

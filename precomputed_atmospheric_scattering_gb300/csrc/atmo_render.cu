@@ -112,6 +112,8 @@ __device__ float4 ScatteringPairs(const float4* __restrict__ tex, const Shape& s
     const float qc = __shfl_sync(0xffffffffu, c, src);
     const float l1 = __shfl_sync(0xffffffffu, L.lerp_nu, src);
     const float wx = odd ? qa : 1.0f - qa;
+    int rows[4];
+    PairRows(s, p, rows);
     const float wr[4] = {(1.0f - qb) * (1.0f - qc), qb * (1.0f - qc), (1.0f - qb) * qc, qb * qc};
     float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
@@ -120,7 +122,7 @@ __device__ float4 ScatteringPairs(const float4* __restrict__ tex, const Shape& s
       const float wn = wx * (node == 0 ? 1.0f - l1 : l1);
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        const float4 t = __ldg(ATMO_CHECKED_PTR(kCheckLutTexel, tex, PairRow(s, p, q), i, texels));
+        const float4 t = __ldg(ATMO_CHECKED_PTR(kCheckLutTexel, tex, rows[q], i, texels));
         const float w = wn * wr[q];
         acc.x = fmaf(t.x, w, acc.x);
         acc.y = fmaf(t.y, w, acc.y);

@@ -1,5 +1,5 @@
 // Host checks of the 4D lookup's texels as two lanes share them
-// (MakePairLookup, PairRow, PairColumn of atmo_device.cuh).
+// (MakePairLookup, PairRows, PairColumn of atmo_device.cuh).
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -64,11 +64,41 @@ int ForLookups(const Shape& s, F f) {
 int Bounds(const Shape& s) {
   return ForLookups(s, [&](const Lookup4& L) {
     const PairLookup p = MakePairLookup(s, L);
+    int rows[4];
+    PairRows(s, p, rows);
     for (int q = 0; q < 4; ++q) {
       for (int node = 0; node < 2; ++node) {
         for (int upper = 0; upper < 2; ++upper) {
-          const long long i = (long long)PairRow(s, p, q) + PairColumn(s, p, node, upper);
+          const long long i = (long long)rows[q] + PairColumn(s, p, node, upper);
           if (i < 0 || i >= s.s_texels()) return false;
+        }
+      }
+    }
+    return true;
+  });
+}
+
+// The texels of nonzero weight are those that a lookup by itself reads
+// (Scattering4: the columns of each node clamped one by one).
+int Texels(const Shape& s) {
+  const int W = s.sw(), H = s.smu, D = s.sr;
+  return ForLookups(s, [&](const Lookup4& L) {
+    const int y = ToInt(std::floor(L.y)), z = ToInt(std::floor(L.z)), x = ToInt(std::floor(L.xl));
+    const float wy = L.y - std::floor(L.y), wz = L.z - std::floor(L.z);
+    const PairLookup p = MakePairLookup(s, L);
+    int rows[4];
+    PairRows(s, p, rows);
+    for (int q = 0; q < 4; ++q) {
+      if (((q & 1) && wy == 0.0f) || ((q & 2) && wz == 0.0f)) continue;
+      if (L.z != L.z || std::isinf(L.z) || L.y != L.y) continue;   // weights are NaN
+      // A view of no finite length: the first column has wrapped.
+      if (std::abs((long long)L.b0) > 1000 * s.smus) continue;
+      const int j = ClampIdx(y + (q & 1), H), k = ClampIdx(z + (q >> 1), D);
+      for (int node = 0; node < 2; ++node) {
+        for (int upper = 0; upper < 2; ++upper) {
+          const int i = ClampIdx((node == 0 ? L.b0 : L.b1) + x + upper, W);
+          if (rows[q] + PairColumn(s, p, node, upper) != (k * H + j) * W + i)
+            return false;
         }
       }
     }
@@ -84,6 +114,7 @@ int main(int argc, char** argv) {
   int bad = 0;
   for (const Shape& s : shapes) {
     if (argc > 1 && std::strcmp(argv[1], "bounds") == 0) bad += Bounds(s);
+    if (argc > 1 && std::strcmp(argv[1], "texels") == 0) bad += Texels(s);
   }
   std::printf("%d wrong\n", bad);
   return bad != 0;

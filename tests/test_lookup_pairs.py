@@ -25,3 +25,10 @@ def test_every_texel_is_in_the_lut(binary):
     """Also for a ray that misses the atmosphere, whose radius has no bound."""
     p = subprocess.run([binary, "bounds"], capture_output=True, text=True, timeout=600)
     assert p.returncode == 0, p.stdout + p.stderr
+
+
+def test_texels_are_those_of_a_lookup_by_itself(binary):
+    """Also where nu is outside its range by rounding, so that a node's columns
+    are clamped."""
+    p = subprocess.run([binary, "texels"], capture_output=True, text=True, timeout=600)
+    assert p.returncode == 0, p.stdout + p.stderr
