@@ -12,6 +12,7 @@
 #include <mutex>
 #include <tuple>
 
+#include "atmo_fork.h"
 #include "atmo_kernels.h"
 #include "atmo_tables.cuh"
 
@@ -384,6 +385,27 @@ atmo_status Program::PrepareFork() {
   return ATMO_OK;
 }
 
+// SideBySide's calls for step `side` on the side stream beside step `main`.
+struct Program::ForkOps {
+  Program& p;
+  size_t side, main;
+  cudaStream_t st;
+  atmo_status Fork() {
+    ATMO_CUDA_TRY(cudaEventRecord(p.ev_fork_, st));
+    ATMO_CUDA_TRY(cudaStreamWaitEvent(p.side_stream_, p.ev_fork_, 0));
+    return ATMO_OK;
+  }
+  atmo_status Side() { return p.LaunchStep(side, p.side_stream_); }
+  atmo_status Main() { return p.LaunchStep(main, st); }
+  atmo_status Join() {
+    cudaError_t e = cudaEventRecord(p.ev_join_, p.side_stream_);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(st, p.ev_join_, 0);
+    if (e == cudaSuccess) return ATMO_OK;
+    cudaStreamSynchronize(p.side_stream_);   // the side stream's work is over at least
+    return CudaFail(e, "joining the side stream");
+  }
+};
+
 atmo_status Program::Launch(cudaStream_t st) {
   for (size_t i = 0; i < steps_.size(); ++i) {
     // Pairs of passes that run side by side, the smaller one on the side
@@ -406,12 +428,8 @@ atmo_status Program::Launch(cudaStream_t st) {
         const size_t side = pair ? i : i + 1, main = pair ? i + 1 : i;
         atmo_status s = PrepareFork();
         if (s != ATMO_OK) return s;
-        ATMO_CUDA_TRY(cudaEventRecord(ev_fork_, st));
-        ATMO_CUDA_TRY(cudaStreamWaitEvent(side_stream_, ev_fork_, 0));
-        if ((s = LaunchStep(side, side_stream_)) != ATMO_OK) return s;
-        ATMO_CUDA_TRY(cudaEventRecord(ev_join_, side_stream_));
-        if ((s = LaunchStep(main, st)) != ATMO_OK) return s;
-        ATMO_CUDA_TRY(cudaStreamWaitEvent(st, ev_join_, 0));
+        ForkOps ops{*this, side, main, st};
+        if ((s = SideBySide(ops)) != ATMO_OK) return s;
         ++i;
         continue;
       }

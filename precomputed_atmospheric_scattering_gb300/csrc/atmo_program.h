@@ -109,6 +109,7 @@ class Program {
   // side stream and the fork / join events of Launch.
   bool fork_ = false;
   atmo_status PrepareFork();             // creates the side stream and events once
+  struct ForkOps;
   cudaStream_t side_stream_ = nullptr;
   cudaEvent_t ev_fork_ = nullptr, ev_join_ = nullptr;
 };
