@@ -107,6 +107,25 @@ ATMO_HD float RootFlushed(float x) {
   return sqrtf(x);
 #endif
 }
+ATMO_HD float RcpFlushed(float x) {
+#ifdef __CUDA_ARCH__
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+#else
+  return 1.0f / x;
+#endif
+}
+// a b clamped to [0, 1], NaN to 0 (one product with the .sat modifier).
+ATMO_HD float MulSat(float a, float b) {
+#ifdef __CUDA_ARCH__
+  float y;
+  asm("mul.rn.sat.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b));
+  return y;
+#else
+  return fminf(fmaxf(a * b, 0.0f), 1.0f);
+#endif
+}
 #ifdef ATMO_FLUSHED_GEOMETRY
 ATMO_HD float quot(float a, float b) { return QuotFlushed(a, b); }
 ATMO_HD float root(float x) { return RootFlushed(x); }
@@ -428,6 +447,37 @@ ATMO_HD float UMuSFromMuS(const Consts& c, const Shape& s, float mu_s) {
   float d_min = c.Rt - c.Rb, d_max = c.H;
   float a = quot(d - d_min, d_max - d_min);
   return TexCoord(s, kMapSMUS, quot(fmaxf(1.0f - quot(a, c.mus_A), 0.0f), 1.0f + a));
+}
+
+// The mu_s mapping along a ray of many samples: with d the distance to the top
+// and a = (d - d_min) / (d_max - d_min), x = (1 - a / A) / (1 + a).  Above the
+// horizon d is H^2 / y, below it y, y = sqrt(H^2 + (Rb mu_s)^2) + |Rb mu_s|
+// (cancellation-free); with g = H^2 - d_min y and y - d_min, x is (b - g k / A) /
+// (b + g k), b = y and 1, k = 1 / (d_max - d_min): one reciprocal.  g keeps the
+// precision of d - d_min, of which x has 1 / A (large where the sun stays high):
+// with x as an FMA of 1 / (1 + a), one instruction less, the scattering LUT's
+// rms error was 12% larger for the Earth, and x's four times at a maximum sun
+// zenith angle of 60 degrees.
+struct SunMap {
+  float H2, d_min, k, k_A;
+  float n1;   // MU_S - 1
+};
+ATMO_HD SunMap MakeSunMap(const Consts& c, const Shape& s) {
+  SunMap m;
+  m.H2 = c.H * c.H;
+  m.d_min = c.Rt - c.Rb;
+  m.k = 1.0f / (c.H - m.d_min);
+  m.k_A = m.k / c.mus_A;
+  m.n1 = float(s.smus - 1);
+  return m;
+}
+// The mapping's x, in [0, 1], where the sun's cosine is rmus / Rb.
+ATMO_HD float SunCoordinate(const SunMap& m, float rmus) {
+  // y >= H and b + g k >= min(1, H): normal.
+  const float y = RootFlushed(fmaf(rmus, rmus, m.H2)) + fabsf(rmus);
+  const bool up = rmus > 0.0f;
+  const float g = fmaf(up ? -m.d_min : 1.0f, y, up ? m.H2 : -m.d_min), b = up ? y : 1.0f;
+  return MulSat(fmaf(-m.k_A, g, b), RcpFlushed(fmaf(m.k, g, b)));
 }
 
 // u_mu when the distance to the ray's boundary is known (d_ray).

@@ -1450,7 +1450,7 @@ __device__ __forceinline__ void MultipleFastBlock(const Instance& in, int local,
 // marches its own columns' tasks needs 1.7.
 //
 // Bound by the L1 data pipe (78%) and instruction issue (74%) together, 27
-// wavefronts and 97 instructions per warp and sample, against 45 and 135 of
+// wavefronts and 98 instructions per warp and sample, against 45 and 135 of
 // the lines in shared memory, whose stores, taps and clamps it does without.
 // Of a sample's four rows those it shares with the last one stay in
 // registers.  Per 16-instance launch at the reference's shape 4.13 (lines in
@@ -1480,37 +1480,6 @@ __host__ __device__ inline int NodeRows(const Shape& s) {
   const bool many = (long long)s.sr * s.smu * items >= 4LL * kNodeWarps * 4 * 152;
   const int rows = (many ? 4 : 1) * kNodeWarps / items;
   return rows < 1 ? 1 : (rows > 4 ? 4 : rows);
-}
-
-// The mu_s mapping along a ray: with a = (d - d_min) / (d_max - d_min) the
-// mapping's x = (1 - a / A) / (1 + a) is ((A + 1) / (1 + a) - 1) / A, one FMA
-// of 1 / (1 + a).
-struct SunMap {
-  float H2, c0, c1, c1h2;   // 1 + a = c0 + c1 d; c1 H^2
-  float k1, k0;             // x = k1 / (1 + a) + k0, clamped to [0, 1]
-  float n1;                 // MU_S - 1
-};
-__device__ __forceinline__ SunMap MakeSunMap(const Consts& c, const Shape& s) {
-  SunMap m;
-  const float d_min = c.Rt - c.Rb, inv_A = 1.0f / c.mus_A;
-  m.H2 = c.H * c.H;
-  m.c1 = 1.0f / (c.H - d_min);
-  m.c0 = 1.0f - d_min * m.c1;
-  m.c1h2 = m.c1 * m.H2;
-  m.k1 = 1.0f + inv_A;
-  m.k0 = -inv_A;
-  m.n1 = float(s.smus - 1);
-  return m;
-}
-// The mapping's x, in [0, 1], where the sun's cosine is rmus / Rb.
-__device__ __forceinline__ float SunCoordinate(const SunMap& m, float rmus) {
-  // H^2 + rmus^2 >= H^2 and y >= H: normal.  d = H^2 / y above the horizon,
-  // y below it (cancellation-free), so 1 / (1 + a) is y / (c0 y + c1 H^2) or
-  // 1 / (c0 + c1 y), both denominators >= min(1, H).
-  const float y = SqrtFtz(fmaf(rmus, rmus, m.H2)) + fabsf(rmus);
-  const bool up = rmus > 0.0f;
-  const float q = DivFtz(up ? y : 1.0f, fmaf(up ? m.c0 : m.c1, y, up ? m.c1h2 : m.c0));
-  return FmaSat(q, m.k1, m.k0);
 }
 
 // LoadIf of two neighbouring texels (32-byte aligned).
