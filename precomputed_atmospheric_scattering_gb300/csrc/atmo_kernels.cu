@@ -16,8 +16,9 @@ namespace atmo {
 // the first blocks and not in every row's last block, whose other threads
 // waited for it at the end.  Per 16-instance
 // launch at the reference's shape 0.568 -> 0.458 ms with the layers in
-// registers and the approximate altitude of OpticalLengthPartial -> 0.426; one
-// instance 49 -> 42 -> 35 us.
+// registers and an approximate altitude, 0.424 with the horizon's rays apart and
+// 0.451 with the altitude as precise as IEEE forms make it (0.475 with these);
+// one instance 49 -> 42 -> 35 -> 37 us.
 __global__ void __launch_bounds__(kTransmittanceThreads, 4)
 k_transmittance(const Instance* __restrict__ insts, WorkList wl) {
   __shared__ HorizonRay horizon[kHorizonTexelsPerTile];

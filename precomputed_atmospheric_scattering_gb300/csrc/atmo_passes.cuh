@@ -142,6 +142,13 @@ ATMO_PASS_COLD F3 TangentDensities(const Consts& c, const HorizonRay& ray, int q
             ProfileDensity64(c.prof_a, h)};
 }
 
+// A sample's radius from its square: the approximate root's product, corrected
+// by its residual (Newton's step for a root).
+ATMO_PASS float SampleRadius(float r2) {
+  const float y = rsqrtf(r2), r = r2 * y;
+  return fmaf(0.5f * y, fmaf(-r, r, r2), r);
+}
+
 // A sample's altitude a / b, b in [2 Rb, 2 Rt]: the approximate reciprocal's
 // product, corrected by its residual (Newton's step for a quotient).
 ATMO_PASS float SampleAltitude(float a, float b) {
@@ -149,11 +156,11 @@ ATMO_PASS float SampleAltitude(float a, float b) {
   return fmaf(fmaf(-h, b, a), y, h);
 }
 
-// The layers are read once and selected from registers, and a sample's radius
-// takes the approximate square root (its error is halved in the altitude).  The
-// LUT's error against 64 bits, mean over 40 atmospheres and sizes, relative: rms
-// 1.0191e-6 (1.0192e-6 with IEEE forms), mean 3.063e-7 (3.066e-7), of the norm
-// 9.42e-8 (9.40e-8); an uncorrected quotient 1.0202e-6, 3.075e-7, 9.51e-8.
+// The layers are read once and selected from registers.  With the corrected root
+// and quotient the LUT's error against 64 bits, mean over 40 atmospheres and
+// sizes, is that of IEEE forms (relative rms 1.0192e-6, mean 3.066e-7, of the
+// norm 9.400e-8); with the approximate root 9.418e-8 of the norm, with neither
+// corrected rms 1.0202e-6, mean 3.075e-7 and 9.51e-8.
 // horizon: the texel's FP64 ray in the horizon column, else null.
 ATMO_PASS void OpticalLengthPartial(const Consts& c, const TransmittanceRay& ray,
                                     const HorizonRay* horizon, int first, int stride,
@@ -165,7 +172,7 @@ ATMO_PASS void OpticalLengthPartial(const Consts& c, const TransmittanceRay& ray
   for (int q = first; q <= kOpticalLengthSamples; q += stride) {
     const float d = float(q) * ray.dx;
     const float rho2 = clampf(fmaf(d, d + 2.0f * ray.rmu, ray.rho * ray.rho), 0.0f, h2);
-    const float h = SampleAltitude(rho2, RootFlushed(rho2 + rb2) + rb);
+    const float h = SampleAltitude(rho2, SampleRadius(rho2 + rb2) + rb);
     float w = (q == 0 || q == kOpticalLengthSamples) ? 0.5f : 1.0f;
     if (horizon && h < near_ground) {
       const F3 density = TangentDensities(c, *horizon, q);
