@@ -141,7 +141,9 @@ typedef enum {
 typedef enum { ATMO_DTYPE_F32 = 0, ATMO_DTYPE_F16 = 1 } atmo_dtype;
 
 typedef struct {
-  void* device_ptr;        /* RGBA texels, x fastest, then y, then z */
+  void* device_ptr;        /* RGBA texels, x fastest, then y, then z; 512-byte
+                              aligned in a model or batch, whose LUTs lie in one
+                              allocation (take offsets from its base for IPC) */
   int width, height, depth;
   atmo_dtype dtype;
   size_t bytes;

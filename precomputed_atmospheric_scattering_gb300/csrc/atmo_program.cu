@@ -77,12 +77,13 @@ atmo_status Storage::Allocate(const Shape& shape, bool combined_textures, bool h
   half = half_precision;
   const size_t nT = (size_t)s.t_texels(), nI = (size_t)s.i_texels(),
                nS = (size_t)s.s_texels();
-  // One allocation, each buffer on a 256-byte boundary: first the offsets.
+  // One allocation: first the offsets, on the 512-byte boundaries that an
+  // allocation of its own has (texture objects on linear memory need them).
   std::vector<std::pair<void**, size_t>> parts;
   size_t total = 0;
   auto place = [&](void** p, size_t bytes) {
     parts.push_back({p, total});
-    total += (bytes + 255) / 256 * 256;
+    total += (bytes + 511) / 512 * 512;
   };
 #define ATMO_ALLOC(ptr, bytes) place(reinterpret_cast<void**>(&(ptr)), (bytes))
   ATMO_ALLOC(T, nT * sizeof(float4));
