@@ -302,8 +302,9 @@ atmo_status atmo_batch_destroy(atmo_batch* batch);
 /* Replaces the parameters of instance i (same shape and order count). */
 atmo_status atmo_batch_set_atmosphere(atmo_batch* batch, unsigned i,
                                       const atmo_atmosphere* atmosphere);
-/* Runs every instance's full precomputation; the pass sequence is captured
-   in a CUDA graph on first use and replayed afterwards. */
+/* Runs every instance's full precomputation.  The first run launches the
+   kernels one by one; the second captures the pass sequence in a CUDA graph,
+   which it and the later runs replay. */
 atmo_status atmo_batch_run(atmo_batch* batch, atmo_stream stream);
 atmo_status atmo_batch_get_lut(const atmo_batch* batch, unsigned i, atmo_lut_kind kind,
                                atmo_lut_view* view);
@@ -314,9 +315,11 @@ atmo_status atmo_batch_read_lut(const atmo_batch* batch, unsigned i, atmo_lut_ki
    ordered on `stream` (make it wait for the run first, e.g. with an event). */
 atmo_status atmo_batch_copy_lut(const atmo_batch* batch, unsigned i, atmo_lut_kind kind,
                                 void* dst, size_t bytes, atmo_stream stream);
-/* Number of kernels one atmo_batch_run launches (for launch accounting). */
+/* Number of kernels one atmo_batch_run launches (for launch accounting): one
+   per pass and kernel variant that the instances' shapes take, and those that
+   carry the launch descriptors. */
 atmo_status atmo_batch_kernel_count(const atmo_batch* batch, unsigned* count);
-/* Runs the batch once without a graph and times every kernel with CUDA
+/* Runs the batch once without a graph and times every pass with CUDA
    events on `stream`: ms[i], pass[i] (0 tables, 1 transmittance, 2 direct
    irradiance, 3 single scattering, 4 scattering density, 5 indirect
    irradiance, 6 multiple scattering, 7 FP16 conversion) and order[i] for

@@ -99,6 +99,10 @@ ATMO_HD int SingleKind(const Shape& s) {
     return s.sw() <= 128 || s.tw > 256 || s.sr * s.smu < 304 ? kSingleOne : kSingleTwo;
   return s.sw() <= 512 ? kSingleTwoWide : kSingleFour;
 }
+// The bits of a pass's kernels; of `kinds`, as many as the pass launches.
+constexpr int kMultipleKinds = 1 | 2 | 4;
+constexpr int kDensityKinds = kDensityArcs4 | kDensityArcs8 | kDensityLookups;
+constexpr int kSingleKinds = kSingleOne | kSingleTwo | kSingleTwoWide | kSingleFour;
 ATMO_HD int KernelKinds(const Shape& s) {
   return MultipleKind(s) | DensityKind(s) | SingleKind(s) |
          (s.sw() > 128 && SingleKind(s) == kSingleOne ? kSingleOneWide : 0);

@@ -310,6 +310,43 @@ __global__ void k_write_descriptors(const __grid_constant__ DescriptorWords d, i
 }
 static_assert(sizeof(Instance) % sizeof(int) == 0, "descriptors are copied as words");
 
+static bool DescriptorsAsWords(size_t bytes) {
+  return bytes <= kMaxWordLaunches * kDescriptorWords * sizeof(int);
+}
+
+int Program::Kinds(const std::pair<int, int>& list) const {
+  int kinds = 0;
+  for (int i = 0; i < list.second; ++i) kinds |= KernelKinds(slots[blob_[list.first + i]].s);
+  return kinds;
+}
+
+int Program::KernelCount() const {
+  auto bits = [](int x) {
+    int n = 0;
+    for (; x != 0; x &= x - 1) ++n;
+    return n;
+  };
+  const size_t words = DescriptorBytes() / sizeof(int);
+  int count =
+      DescriptorsAsWords(DescriptorBytes()) ? (int)((words + kDescriptorWords - 1) / kDescriptorWords)
+                                            : 0;
+  for (const Step& step : steps_) {
+    const auto& list = wl_offsets_[step.wl];
+    const bool fast = step.path == ATMO_PATH_FAST;
+    int kinds = 0;   // 0: one kernel whatever the instances
+    if (fast && step.pass == Pass::kSingle) kinds = Kinds(list) & kSingleKinds;
+    if (fast && step.pass == Pass::kMultiple) kinds = Kinds(list) & kMultipleKinds;
+    if (fast && step.pass == Pass::kDensity && step.order > 2) kinds = Kinds(list) & kDensityKinds;
+    if (step.pass == Pass::kToHalf) {
+      const Instance& in = slots[blob_[list.first]];
+      count += (in.S_half != nullptr) + (in.M && in.M_half);
+    } else {
+      count += kinds != 0 ? bits(kinds) : 1;
+    }
+  }
+  return count;
+}
+
 atmo_status Program::Finalize() {
   if (finalized_) return ATMO_OK;
   if (!d_slots_) {
@@ -323,11 +360,10 @@ atmo_status Program::Finalize() {
     w.inst = lists + o.first;
     w.start = lists + o.first + o.second;
     w.count = o.second;
-    w.kinds = 0;
-    for (int i = 0; i < o.second; ++i) w.kinds |= KernelKinds(slots[blob_[o.first + i]].s);
+    w.kinds = Kinds(o);
     wls_.push_back(w);
   }
-  if (DescriptorBytes() > kMaxWordLaunches * kDescriptorWords * sizeof(int))
+  if (!DescriptorsAsWords(DescriptorBytes()))
     ATMO_CUDA_TRY(cudaMallocHost(&h_pinned_, DescriptorBytes()));
   // Row orders of the instances that have the table (slots of one model share
   // it; the radii of a later set_atmosphere leave the order stale, which

@@ -86,13 +86,15 @@ class Program {
   // Upload + launch; with use_graph, the second and later runs replay a CUDA
   // graph.
   atmo_status Run(cudaStream_t st, bool use_graph);
-  int KernelCount() const { return (int)steps_.size(); }
+  // Kernels of one run, the descriptors' among them.
+  int KernelCount() const;
   std::vector<Step> const& steps() const { return steps_; }
 
  private:
   int AddWorkList(const std::vector<int>& members, Pass pass, int order, int* tiles,
                   int* smem = nullptr, atmo_path* step_path = nullptr);
   std::vector<Step> steps_;
+  int Kinds(const std::pair<int, int>& list) const;   // of a work list's instances
   std::vector<int> blob_;              // inst[] then start[] of every work list
   std::vector<std::pair<int, int>> wl_offsets_;  // (offset, count)
   std::vector<WorkList> wls_;
