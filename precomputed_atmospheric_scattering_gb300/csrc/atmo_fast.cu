@@ -1796,12 +1796,14 @@ int MultipleFastTiles(const Shape& s) {
   const int rows = MultipleByNodes(s) ? NodeRows(s) : MultipleDims(s).rows;
   return (s.sr * s.smu + rows - 1) / rows;
 }
-int MultipleFastSmem(const Shape& s) {
-  if (MultipleByNodes(s))
-    return NodeRows(s) * (kNodeSamples * (int)sizeof(RaySample) + 4 * s.smus * 16) +
-           kNodeWarps * 96 * MultipleKind(s) * (int)sizeof(NodeTask);
+static int MultipleLinesSmem(const Shape& s) {
   const MultipleFastDims d = MultipleDims(s);
   return d.rows * kRaySamples * (int)sizeof(RaySample) + 2 * d.group * d.rows * s.sw() * 16;
+}
+int MultipleFastSmem(const Shape& s) {
+  if (!MultipleByNodes(s)) return MultipleLinesSmem(s);
+  return NodeRows(s) * (kNodeSamples * (int)sizeof(RaySample) + 4 * s.smus * 16) +
+         kNodeWarps * 96 * MultipleKind(s) * (int)sizeof(NodeTask);
 }
 
 cudaError_t LaunchMultipleFast(const Instance* insts, WorkList wl, int tiles, int smem_bytes,
@@ -1884,7 +1886,8 @@ int SingleFastTiles(const Shape& s) {
 
 // Whether a (rows, group) block shape is launchable for shape s: one texel
 // column per thread needs rows x W <= 256 (wider rows take one row per
-// block), and the shared memory must stay within 48 KB.
+// block), and the shared memory of the lines must stay within 48 KB (of the
+// shapes without lines too: a tuning is valid or not whichever kernel is taken).
 bool FastTuningValid(const Shape& s, bool single, int rows, int group) {
   if (rows < 1 || rows > 4 || group < 1 || group > 8) return false;
   const int W = s.sw();
@@ -1893,7 +1896,7 @@ bool FastTuningValid(const Shape& s, bool single, int rows, int group) {
   Shape t = s;
   t.tune[single ? 2 : 0] = rows;
   t.tune[single ? 3 : 1] = group;
-  return (single ? SingleFastLimit(t) : MultipleFastSmem(t)) <= 48 * 1024;
+  return (single ? SingleFastLimit(t) : MultipleLinesSmem(t)) <= 48 * 1024;
 }
 
 // Sample i of the ray of LUT row `rowi` (the per-sample part of
