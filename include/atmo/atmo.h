@@ -488,9 +488,9 @@ atmo_status atmo_server_get_stats(atmo_server* server, atmo_server_stats* out);
    for one LUT shape: scattering-LUT rows per block and ray samples per
    shared-memory line stage (0, 0: the built-in choice; shapes whose multiple
    scattering needs no shared-memory lines take the same blocks under every
-   multiple_* value; single scattering takes at most 128 columns' rows per
-   block).  A tuning changes only how work is grouped: every LUT is
-   bit-identical under every tuning. */
+   multiple_* value, and the autotuner gives 1, 1; single scattering takes at
+   most 128 columns' rows per block).  A tuning changes only how work is
+   grouped: every LUT is bit-identical under every tuning. */
 typedef struct {
   int multiple_rows, multiple_group;
   int single_rows, single_group;

@@ -1213,8 +1213,19 @@ atmo_status atmo_autotune(const atmo_atmosphere* atmosphere, const atmo_lut_shap
   const int rows_c[3] = {1, 2, 4}, group_c[6] = {1, 2, 3, 4, 6, 8};
   for (int r : rows_c) {
     for (int g : group_c) {
-      const bool ms_ok = FastTuningValid(base, false, r, g);
-      const bool ss_ok = FastTuningValid(base, true, r, g);
+      // Each launch once: of the rows that come to the same, and of all where
+      // the kernel takes no tuning, the first.
+      auto fresh = [&](bool single) {
+        if (!FastTuningValid(base, single, r, g)) return false;
+        const int rows = FastTuningRows(base, single, r);
+        if (rows == 0) return trials.empty();
+        for (int earlier : rows_c)
+          if (earlier < r && FastTuningValid(base, single, earlier, g) &&
+              FastTuningRows(base, single, earlier) == rows)
+            return false;
+        return true;
+      };
+      const bool ms_ok = fresh(false), ss_ok = fresh(true);
       if (!ms_ok && !ss_ok) continue;
       Shape s = base;
       s.tune[0] = ms_ok ? r : 0;

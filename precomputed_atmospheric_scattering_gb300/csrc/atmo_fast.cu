@@ -1899,6 +1899,13 @@ bool FastTuningValid(const Shape& s, bool single, int rows, int group) {
   return (single ? SingleFastLimit(t) : MultipleLinesSmem(t)) <= 48 * 1024;
 }
 
+int FastTuningRows(const Shape& s, bool single, int rows) {
+  if (!single) return MultipleByNodes(s) ? 0 : rows;
+  Shape t = s;
+  t.tune[2] = rows;
+  return SingleDims(t, kSingleThreads).rows;
+}
+
 // Sample i of the ray of LUT row `rowi` (the per-sample part of
 // SingleScatteringTexel that does not depend on mu_s or nu).
 __device__ SunSample MakeSunSample(const Instance& in, int rowi, int i) {

@@ -41,6 +41,8 @@ cudaError_t LaunchSingleFast(const Instance* insts, WorkList wl, int tiles, int 
 // A (rows per block, samples per line stage) tuning of the single (single =
 // true) or multiple scattering kernel that can run for shape s.
 bool FastTuningValid(const Shape& s, bool single, int rows, int group);
+// The rows per block that a valid tuning comes to (0: the kernel takes none).
+int FastTuningRows(const Shape& s, bool single, int rows);
 // The row-restructured multiple-scattering kernel needs W = NU x MU_S <= 1024.
 bool MultipleFastFits(const Shape& s);
 int MultipleFastTiles(const Shape& s);
