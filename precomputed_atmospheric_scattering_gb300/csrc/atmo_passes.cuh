@@ -206,7 +206,8 @@ ATMO_PASS F3 DirectIrradianceTexel(const Instance& in, int texel) {
   IrrRow row = in.tab.irows[j];
   float mu_s = in.tab.mus_i[i];
   float a = c.alpha_s;
-  float f = mu_s < -a ? 0.0f : (mu_s > a ? mu_s : (mu_s + a) * (mu_s + a) / (4.0f * a));
+  // Zero at mu_s = -a too, where a point sun's quotient would be 0 / 0.
+  float f = mu_s <= -a ? 0.0f : (mu_s > a ? mu_s : (mu_s + a) * (mu_s + a) / (4.0f * a));
   return c.solar * TransmittanceToTop(c, s, in.T, row.rho, row.r, row.r * mu_s) * f;
 }
 
