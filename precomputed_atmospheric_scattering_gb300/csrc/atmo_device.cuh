@@ -126,11 +126,14 @@ ATMO_HD float MulSat(float a, float b) {
   return fminf(fmaxf(a * b, 0.0f), 1.0f);
 #endif
 }
+// unit_quot: a quotient in [0, 1]; 0 where flushing makes it 0 / 0.
 #ifdef ATMO_FLUSHED_GEOMETRY
 ATMO_HD float quot(float a, float b) { return QuotFlushed(a, b); }
+ATMO_HD float unit_quot(float a, float b) { return MulSat(a, RcpFlushed(b)); }
 ATMO_HD float root(float x) { return RootFlushed(x); }
 #else
 ATMO_HD float quot(float a, float b) { return a / b; }
+ATMO_HD float unit_quot(float a, float b) { return a / b; }
 ATMO_HD float root(float x) { return sqrtf(x); }
 #endif
 
@@ -140,7 +143,7 @@ ATMO_HD float clampf(float x, float lo, float hi) { return fminf(fmaxf(x, lo), h
 ATMO_HD float smoothstepf(float e0, float e1, float x) {
   if (x <= e0) return 0.0f;
   if (x >= e1) return 1.0f;
-  float t = quot(x - e0, e1 - e0);
+  float t = unit_quot(x - e0, e1 - e0);   // subnormal operands: flushed, to 0 / 0
   return t * t * (3.0f - 2.0f * t);
 }
 
