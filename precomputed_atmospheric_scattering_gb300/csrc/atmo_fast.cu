@@ -1450,7 +1450,7 @@ __device__ __forceinline__ void MultipleFastBlock(const Instance& in, int local,
 // marches its own columns' tasks needs 1.7.
 //
 // Bound by the L1 data pipe (78%) and instruction issue (74%) together, 27
-// wavefronts and 98 instructions per warp and sample, against 45 and 135 of
+// wavefronts and 99 instructions per warp and sample, against 45 and 135 of
 // the lines in shared memory, whose stores, taps and clamps it does without.
 // Of a sample's four rows those it shares with the last one stay in
 // registers.  Per 16-instance launch at the reference's shape 4.13 (lines in

@@ -320,28 +320,30 @@ int Program::Kinds(const std::pair<int, int>& list) const {
   return kinds;
 }
 
+int PassKernels(Pass pass, int order, atmo_path path, int kinds) {
+  int of = 0;   // 0: one kernel whatever the instances
+  if (path == ATMO_PATH_FAST) {
+    if (pass == Pass::kSingle) of = kinds & kSingleKinds;
+    if (pass == Pass::kMultiple) of = kinds & kMultipleKinds;
+    if (pass == Pass::kDensity && order > 2) of = kinds & kDensityKinds;
+  }
+  int n = 0;
+  for (; of != 0; of &= of - 1) ++n;
+  return n > 0 ? n : 1;
+}
+
 int Program::KernelCount() const {
-  auto bits = [](int x) {
-    int n = 0;
-    for (; x != 0; x &= x - 1) ++n;
-    return n;
-  };
   const size_t words = DescriptorBytes() / sizeof(int);
   int count =
       DescriptorsAsWords(DescriptorBytes()) ? (int)((words + kDescriptorWords - 1) / kDescriptorWords)
                                             : 0;
   for (const Step& step : steps_) {
     const auto& list = wl_offsets_[step.wl];
-    const bool fast = step.path == ATMO_PATH_FAST;
-    int kinds = 0;   // 0: one kernel whatever the instances
-    if (fast && step.pass == Pass::kSingle) kinds = Kinds(list) & kSingleKinds;
-    if (fast && step.pass == Pass::kMultiple) kinds = Kinds(list) & kMultipleKinds;
-    if (fast && step.pass == Pass::kDensity && step.order > 2) kinds = Kinds(list) & kDensityKinds;
     if (step.pass == Pass::kToHalf) {
       const Instance& in = slots[blob_[list.first]];
       count += (in.S_half != nullptr) + (in.M && in.M_half);
     } else {
-      count += kinds != 0 ? bits(kinds) : 1;
+      count += PassKernels(step.pass, step.order, step.path, Kinds(list));
     }
   }
   return count;

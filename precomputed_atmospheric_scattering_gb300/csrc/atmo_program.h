@@ -123,6 +123,8 @@ atmo_path PassPath(Pass pass, const Shape& s, atmo_path path);
 // Blocks and dynamic shared memory of `pass` for shape s under the variant
 // `path` (as PassPath returns it).
 int Tiles(Pass pass, const Shape& s, atmo_path path, int order);
+// Kernels that LaunchPass launches for a work list of these kinds.
+int PassKernels(Pass pass, int order, atmo_path path, int kinds);
 // Dynamic shared memory of a pass's launch for one instance (shape and
 // constants: the density pass sizes its merged tables from the radii).
 int SharedBytes(Pass pass, const Shape& s, const Consts& c, int order, atmo_path path);

@@ -497,7 +497,7 @@ bool atmo_server::LaunchRound() {
   for (const Launch& l : launches) {
     if (e != cudaSuccess) break;
     e = LaunchPass(l.pass, l.order, l.smem, d_inst, l.wl, l.tiles, l.path, build_stream);
-    ++stats.kernels;
+    stats.kernels += PassKernels(l.pass, l.order, l.path, l.wl.kinds);
   }
   if (e != cudaSuccess) {
     worker_error = std::string("round launch: ") + cudaGetErrorString(e);
