@@ -1456,7 +1456,7 @@ __device__ __forceinline__ void MultipleFastBlock(const Instance& in, int local,
 // registers.  Per 16-instance launch at the reference's shape 4.13 (lines in
 // shared memory) -> 3.25 (nodes) -> 3.08 (packed tasks) -> 2.95 (four items
 // per warp, handed out) -> 2.76 ms (shared rows kept); one high-resolution
-// instance 4.40 -> 3.43 -> 3.08 -> 3.03 -> 2.73 ms.
+// instance 4.40 -> 3.43 -> 3.08 -> 3.03 -> 2.72 ms.
 // ---------------------------------------------------------------------------
 constexpr int kNodeWarps = kMultipleFastThreads / 32;
 constexpr int kNodeSamples = kRaySamples + 1;   // the last one twice
@@ -1470,14 +1470,14 @@ __host__ __device__ inline int NodeItemsPerRow(const Shape& s) {
   return (s.snu + per - 1) / per;
 }
 // Rows per block: as many (up to 4) as give its 8 warps one item each, or four
-// where that leaves a full wave of blocks (4 per SM on 152 SMs).  Four items
+// where that leaves a full wave of blocks (4 per SM).  Four items
 // per warp shorten the blocks' idle time (their sample tables are built by 51
 // threads per row, and the items differ): 2.82 ms per 16-instance launch at
 // the reference's shape against 2.91 with two; smaller LUTs want the shorter
 // blocks.
 __host__ __device__ inline int NodeRows(const Shape& s) {
   const int items = NodeItemsPerRow(s);
-  const bool many = (long long)s.sr * s.smu * items >= 4LL * kNodeWarps * 4 * 152;
+  const bool many = (long long)s.sr * s.smu * items >= 4LL * kNodeWarps * 4 * kSmCount;
   const int rows = (many ? 4 : 1) * kNodeWarps / items;
   return rows < 1 ? 1 : (rows > 4 ? 4 : rows);
 }
@@ -2146,7 +2146,7 @@ cudaError_t LaunchSingleFast(const Instance* insts, WorkList wl, int tiles, int 
     // without a texel column help with the samples and the lines: one instance
     // of half size (1024 rows of 64 columns) 43 us against 51; 8 of them 260
     // us against 234.  Rows of more than 128 columns need them.
-    const bool all = tiles <= 4 * 152 || wl.kinds & kSingleOneWide;
+    const bool all = tiles <= 4 * kSmCount || wl.kinds & kSingleOneWide;
     k_single_fast<kSingleOne><<<tiles, all ? kMultipleFastThreads : kSingleThreads, bytes, st>>>(
         insts, wl, kRoundMagic);
   }

@@ -46,6 +46,8 @@ struct WorkList {
   int kinds;   // the instances' KernelKinds bits
 };
 
+constexpr int kSmCount = 152;   // of a GB300
+
 // The multiple-scattering kernel of a LUT shape, a bit: 1, the mu_s columns of
 // a nu node in one register per lane (MU_S <= 32); 2, in two (MU_S 33 to 64);
 // 4, lines in shared memory.  The nodes win unless many lanes idle: kernel 4
@@ -91,7 +93,9 @@ ATMO_HD int DensityKind(const Shape& s) {
 // a row of up to 128 columns has only one for each thread (64 columns, one
 // instance: 57 us, with two 76), and a row of wide transmittance lines, or of a
 // LUT of few rows, wants 256 threads to build the lines (204 columns, lines of
-// 339: 100 us against 150; 80 rows of 252 columns: 29 us against 31).
+// 339: 100 us against 150; 80 rows of 252 columns: 29 us against 31).  Of 69 shapes
+// of 24 to 1024 columns one loses against 16-byte line entries built row by row:
+// 442 rows of 64 x 12 columns take 6% longer (18% less on average).
 constexpr int kSingleOne = 64, kSingleTwo = 128, kSingleTwoWide = 256, kSingleFour = 512;
 constexpr int kSingleOneWide = 1024;   // with kSingleOne: needs 256 threads
 ATMO_HD int SingleKind(const Shape& s) {
